@@ -220,7 +220,7 @@ def branch_flows(net: Network, v, base_power, taps=True, i_n=None, sn=None, bran
     bst = net.n_branch * 6 if br.dim() == 3 else 0
     inn = None if i_n is None else torch.as_tensor(np.asarray(i_n, np.float64), device=dev)
     snn = None if sn is None else torch.as_tensor(np.asarray(sn, np.float64), device=dev)
-    out = torch.zeros((S, net.n_branch, 9), dtype=torch.float64, device=dev)
+    out = torch.empty((S, net.n_branch, 9), dtype=torch.float64, device=dev)  # every row written
     N.check(N.lib().gapk_branch_flows(S, net.n_bus, net.n_branch, _dptr(fi), _dptr(ti),
                                       _dptr(br), bst, _dptr(v), float(base_power),
                                       float(net.u_rated[0]), _dptr(inn), _dptr(snn),

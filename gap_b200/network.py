@@ -107,9 +107,8 @@ class Network:
         IDs, later duplicates overwrite earlier ones, negative IDs are never mapped."""
         max_id = int(self.bus_id.max()) if self.n_bus else -1
         lut = np.full(max_id + 1, -1, dtype=np.int64)
-        for idx, bid in enumerate(self.bus_id.tolist()):
-            if 0 <= bid <= max_id:
-                lut[bid] = idx
+        pos = np.nonzero(self.bus_id >= 0)[0]
+        lut[self.bus_id[pos]] = pos  # of a repeated ID, the last assignment stays
         return lut
 
     def branch_index(self):
@@ -136,18 +135,11 @@ class Network:
         """(bus_idx, g1, b1) of every SHUNT appliance the reference stamps into the Y-bus
         diagonal (cpu_admittance_matrix.cpp:88-97: all SHUNTs, whatever their status)."""
         lut = self.id_to_index()
-        max_id = lut.shape[0] - 1
-        sel = []
-        for a in range(self.n_app):
-            if self.app_type[a] != SHUNT:
-                continue
-            node = int(self.app_node[a])
-            if 0 <= node <= max_id:
-                bi = int(lut[node])
-                if 0 <= bi < self.n_bus:
-                    sel.append((a, bi))
-        idx = np.array([s[1] for s in sel], dtype=np.int64)
-        aa = np.array([s[0] for s in sel], dtype=np.int64)
+        aa = np.nonzero(self.app_type == SHUNT)[0]
+        node = self.app_node[aa].astype(np.int64)
+        known = (node >= 0) & (node < lut.shape[0])
+        aa, idx = aa[known], lut[node[known]]
+        aa, idx = aa[idx >= 0], idx[idx >= 0]
         return idx, self.app_g1[aa] if len(aa) else np.zeros(0), \
             self.app_b1[aa] if len(aa) else np.zeros(0)
 
@@ -158,13 +150,15 @@ class Network:
         bus ID, divided by base_power when base_power > 0."""
         s = (self.p + 1j * self.q).astype(np.complex128)
         if self.n_app:
+            power = np.nonzero((self.app_status == 1) & ((self.app_type == SOURCE) |
+                                                         (self.app_type == LOADGEN)))[0]
             first = {}
-            for i, bid in enumerate(self.bus_id.tolist()):
-                first.setdefault(bid, []).append(i)
-            for a in range(self.n_app):
-                if self.app_status[a] == 1 and self.app_type[a] in (SOURCE, LOADGEN):
-                    for i in first.get(int(self.app_node[a]), []):
-                        s[i] += complex(self.app_p[a], self.app_q[a])
+            if len(power):
+                for i, bid in enumerate(self.bus_id.tolist()):
+                    first.setdefault(bid, []).append(i)
+            for a in power:
+                for i in first.get(int(self.app_node[a]), []):
+                    s[i] += complex(self.app_p[a], self.app_q[a])
         if base_power > 0.0:
             # component-wise, as std::complex<double> /= double does
             s = (s.real / base_power) + 1j * (s.imag / base_power)
