@@ -101,7 +101,9 @@ __device__ __forceinline__ Blk<T> inv2(Blk<T> const& X, bool& ok) {
     const T tol = T(1e-14);
     const T fa = fabs(X.a), fc = fabs(X.c);
     const T p1 = fa >= fc ? fa : fc;
-    const T schur = fa >= fc ? X.d - X.c * (X.b / X.a) : X.b - X.a * (X.d / X.c);
+    // one division for either pivot row: the other row's remainder
+    const bool top = fa >= fc;
+    const T schur = (top ? X.d : X.b) - (top ? X.c : X.a) * ((top ? X.b : X.d) / (top ? X.a : X.c));
     const T det = X.a * X.d - X.b * X.c;
     ok = p1 >= tol && fabs(schur) >= tol && isfinite(det) && det != T(0);
     if (!ok) return X;

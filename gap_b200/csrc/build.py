@@ -46,7 +46,8 @@ def _run(cmd):
 
 
 CORE_SOURCES = ["symbolic.cpp", "nr.cu", "ybus.cu"]
-HEADERS = ["internal.h", "blocks.cuh", "nr_kernels.cuh", "dense_lu_tc.cuh"]
+HEADERS = ["internal.h", "blocks.cuh", "nr_kernels.cuh", "nr_small.cuh",
+           "dense_lu_tc.cuh"]
 
 
 def build(verbose: bool = False, force: bool = False) -> str:

@@ -2,6 +2,7 @@
 // iteration loop (CUDA graph with a conditional while node), and the gapk_nr_* C ABI.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <memory>
@@ -14,6 +15,7 @@
 #include "../../include/gapk.h"
 #include "internal.h"
 #include "nr_kernels.cuh"
+#include "nr_small.cuh"
 
 namespace gapk {
 
@@ -69,12 +71,95 @@ using namespace gapk;
 struct gapk_nr_plan_s {
     NRPlanHost h;
     std::vector<int> y_row_ptr, y_col;
+    bool general = false;  // the plan of a general LU, not of a Newton solve
     // device copy (current device at first upload)
     bool uploaded = false;
     int device = -1;
-    DevBuf d_yrp, d_ycol, d_bt, d_nob, d_si, d_ss, d_sa, d_lp, d_ln, d_fa, d_tg, d_pr, d_fb,
-        d_sc, d_lptr, d_lidx, d_rptr, d_rl, d_arp, d_ar, d_var, d_eq, d_schur, d_aslots, d_acp, d_ac;
+    DevBuf d_yrp, d_ycol, d_bt, d_nob, d_si, d_ss, d_lp, d_ln, d_fa, d_tg, d_pr, d_fb,
+        d_sc, d_lptr, d_lidx, d_rptr, d_rl, d_arp, d_ar, d_var, d_eq, d_schur, d_aslots, d_arec, d_levels, d_words, d_ell, d_acp, d_ac;
     PlanDev dev{};
+
+    // the Jacobian fill's records (jac_block), four ints per block
+    std::vector<int> a_records() const {
+        std::vector<int> r(4 * (size_t)h.n_a);
+        auto bus = [&](int i) { return i | (h.bus_type[i] == BUS_PQ ? REC_PQ : 0); };
+        for (int a = 0; a < h.n_a; ++a) {
+            const int slot = h.a_slots[a];
+            const int* si = &h.slot_info[4 * (size_t)slot];
+            r[4 * (size_t)a] = slot;
+            r[4 * (size_t)a + 1] = bus(si[0]);
+            r[4 * (size_t)a + 2] = bus(si[1]);
+            r[4 * (size_t)a + 3] = si[3] - si[2] == 1 ? h.slot_src[si[2]] : -1;
+        }
+        return r;
+    }
+
+    // k_nr_small's packed schedule (SmallCta): false when not even one FP32 scenario fits its shared
+    // memory, its 16-bit indices or its tail, and for a general matrix.  Threads per target or row (1, 2 or 4): a pass over two entries costs about 70
+    // cycles of latency, adding up two threads' parts about 45, so the longest row decides where
+    // the level leaves threads idle; a wide level keeps a thread per row.
+    bool small_schedule(std::vector<int>& rec, std::vector<unsigned>& words,
+                        std::vector<unsigned>& ell) const {
+        if (general || h.n_slots > 0xffff || h.nb > 0xffff || h.n_tail > SMALL_MAX_TAIL ||
+            small_layout(h.n_bus, h.nb, h.n_slots, h.n_tail, h.n_levels, 1, 4).total > SMALL_SMEM_MAX)
+            return false;
+        // rows [0, rows) of count(r) words word(r, i), two words to an entry, padded to the
+        // longest part with `pad`; returns (first entry, entries of the longest part | split << 16)
+        auto lists = [&](int rows, auto count, auto word, unsigned pad, int* out) {
+            int most = 0;
+            for (int r = 0; r < rows; ++r) most = std::max(most, count(r));
+            const int ls = rows <= 64 && most > 4 ? 2 : rows <= 128 && most > 2 ? 1 : 0;
+            const int s = 1 << ls, longest = (most + 2 * s - 1) / (2 * s);
+            out[0] = (int)(ell.size() / 2);
+            out[1] = longest | ls << 16;
+            for (int m = 0; m < longest; ++m)
+                for (int r = 0; r < rows; ++r)
+                    for (int sub = 0; sub < s; ++sub)
+                        for (int o = 0; o < 2; ++o) {
+                            const int i = (2 * m + o) * s + sub;
+                            ell.push_back(i < count(r) ? word(r, i) : pad);
+                        }
+        };
+        auto pack = [](int lo, int hi) { return (unsigned)lo | (unsigned)hi << 16; };
+        const unsigned none = pack(h.n_slots, h.n_slots), no_row = pack(h.n_slots, h.nb);
+        rec.assign(12 * ((size_t)h.n_levels + 1), 0);
+        for (int l = 0; l <= h.n_levels; ++l) {
+            const bool tail = l == h.n_levels;
+            int* q = &rec[12 * (size_t)l];
+            const int lb = tail ? h.ns : h.level_ptr[l], c = tail ? h.n_tail : h.level_ptr[l + 1] - lb;
+            q[0] = lb;
+            q[1] = c;
+            if (!tail) {
+                const int t0 = h.fa_ptr[l], nt = h.fa_ptr[l + 1] - t0;
+                const int* tg = &h.targets[4 * (size_t)t0];
+                q[2] = (int)words.size();
+                q[3] = nt;
+                for (int t = 0; t < nt; ++t)
+                    words.push_back((unsigned)tg[4 * t] | (tg[4 * t + 3] & 1 ? SMALL_DIAG : 0) |
+                                  (tg[4 * t + 3] & 2 ? SMALL_VALUE : 0));
+                lists(nt, [&](int t) { return tg[4 * t + 2] - tg[4 * t + 1]; },
+                      [&](int t, int i) {
+                          const int* p = &h.pairs[2 * (size_t)(tg[4 * t + 1] + i)];
+                          return pack(p[0], p[1]);
+                      }, none, q + 4);
+                q[6] = (int)words.size();
+                q[7] = h.fb_ptr[l + 1] - h.fb_ptr[l];
+                for (int t = h.fb_ptr[l]; t < h.fb_ptr[l + 1]; ++t)
+                    words.push_back(pack(h.scale[2 * (size_t)t], h.scale[2 * (size_t)t + 1]));
+                lists(c, [&](int r) { return h.lptr[lb + r + 1] - h.lptr[lb + r]; },
+                      [&](int r, int i) {
+                          const int p = h.lptr[lb + r] + i;
+                          return pack(h.nb + h.nnz_l + p, h.lidx[p]);
+                      }, no_row, q + 10);
+            }
+            lists(c, [&](int r) { return h.rptr[lb + r + 1] - h.rptr[lb + r]; },
+                  [&](int r, int i) {
+                      const int* p = &h.rlist[2 * (size_t)(h.rptr[lb + r] + i)];
+                      return pack(p[0], p[1]);
+                  }, no_row, q + 8);
+        }
+        return true;
+    }
 
     int upload() {
         if (uploaded) return GAPK_OK;
@@ -88,7 +173,6 @@ struct gapk_nr_plan_s {
         up(d_nob, h.node_of_bus);
         up(d_si, h.slot_info);
         up(d_ss, h.slot_src);
-        up(d_sa, h.slot_a);
         up(d_lp, h.level_ptr);
         up(d_ln, h.level_nodes);
         up(d_fa, h.fa_ptr);
@@ -106,6 +190,14 @@ struct gapk_nr_plan_s {
         up(d_eq, h.eq_of_comp);
         up(d_schur, h.schur);
         up(d_aslots, h.a_slots);
+        up(d_arec, a_records());
+        std::vector<int> rec;
+        std::vector<unsigned> words, ell;
+        if (small_schedule(rec, words, ell)) {
+            up(d_levels, rec);
+            if (!rc) rc = d_words.upload(words);
+            if (!rc) rc = d_ell.upload(ell);
+        }
         up(d_acp, h.acol_ptr);
         up(d_ac, h.acol);
         if (rc) return rc;
@@ -123,6 +215,10 @@ struct gapk_nr_plan_s {
         dev.n_schur = static_cast<int>(h.schur.size() / 4);
         dev.schur = d_schur.as<int4>();
         dev.a_slots = d_aslots.as<int>();
+        dev.a_rec = d_arec.as<int4>();
+        dev.levels = d_levels.as<int4>();
+        dev.words = d_words.as<unsigned>();
+        dev.ell = d_ell.as<uint2>();
         dev.acol_ptr = d_acp.as<int>();
         dev.acol = d_ac.as<int2>();
         dev.y_row_ptr = d_yrp.as<int>();
@@ -131,7 +227,6 @@ struct gapk_nr_plan_s {
         dev.node_of_bus = d_nob.as<int>();
         dev.slot_info = d_si.as<int4>();
         dev.slot_src = d_ss.as<int>();
-        dev.slot_a = d_sa.as<int>();
         dev.level_ptr = d_lp.as<int>();
         dev.level_nodes = d_ln.as<int>();
         dev.fa_ptr = d_fa.as<int>();
@@ -150,6 +245,10 @@ struct gapk_nr_plan_s {
     }
 };
 
+struct SmallRun {
+    int cl = 0, threads = 0, together = 0, carveout = 100;
+};
+
 struct gapk_nr_batch_s {
     gapk_nr_plan plan = nullptr;
     int n_scen = 0, sw = 8, G = 0, precision = 0, y_shared = 1, threads = 256, use_graph = 1;
@@ -166,6 +265,8 @@ struct gapk_nr_batch_s {
     cudaGraphExec_t exec = nullptr;
     int graph_refine = -1;
     int cur_refine = 0;
+    SmallRun cur_small;  // how the last inputs' solve runs
+    int wait_test = 0;   // the tensor-core LU's wait test is on
     ~gapk_nr_batch_s() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
@@ -230,7 +331,9 @@ void launch_load(gapk_nr_batch b, const gapk_nr_inputs* in, cudaStream_t st) {
     k_load<SW><<<g, 256, 0, st>>>(P, b->dev, reinterpret_cast<const double2*>(in->d_y),
                                   reinterpret_cast<const double2*>(in->d_s_spec),
                                   reinterpret_cast<const double2*>(in->d_v_init), in->d_u_pu,
-                                  in->v_init_shared);
+                                  in->v_init_shared,
+                                  SolveOpts{1, in->max_iterations, in->policy, in->tolerance,
+                                            in->refine_below, in->reuse_below});
 }
 
 template <int SW>
@@ -490,34 +593,81 @@ int validate_inputs(gapk_nr_batch b, const gapk_nr_inputs* in) {
     return GAPK_OK;
 }
 
+// How the one-kernel loop (k_nr_small) runs this batch on these inputs: lanes per CTA (0: the
+// separate kernels are used), CTA size, whether a group's lanes decide together, and the shared
+// memory share of the SM.  Shapes are ranked by waves of CTAs, then by fewer lanes per CTA (a
+// lane more in a CTA lengthens every step of the level schedule), then by 256 threads over 128.
+// Against the separate kernels on transmission grids of 120 to 1,200 buses it takes 1/1.6 to 1/2.7
+// of their time while one wave holds the scenarios, 1/1.1 to 1/2.2 with two; with three waves it
+// still wins with FP32 factors (1/1.1 to 1/1.25) and where a CTA has an SM to itself (1/1.1), and
+// loses otherwise (300 buses x 1024 scenarios in FP64: 1051 us against 907).
+SmallRun small_choice(gapk_nr_batch b, const gapk_nr_inputs* in) {
+    auto const& h = b->plan->h;
+    SmallRun r;
+    if (b->dev.lvl_ts || b->wait_test || !b->plan->dev.levels) return r;
+    const size_t esz = b->precision == GAPK_PREC_FP64 ? 8 : 4;
+    r.together = in->refine > 0 && (in->refine_below > 0.0 || in->reuse_below > 0.0);
+    long best_cost = 0;
+    for (int cl = 1; cl <= b->sw; cl *= 2) {
+        const size_t bytes = small_layout(h.n_bus, h.nb, h.n_slots, h.n_tail, h.n_levels, cl, esz).total;
+        if (bytes > SMALL_SMEM_MAX) break;
+        for (int thr : {256, 128}) {
+            const long per_cta = (long)bytes + 2048;  // with its static and reserved shared memory
+            const long per_sm = std::min<long>(1024 / thr, SMALL_SM_SMEM / per_cta);
+            const long ctas = ((long)b->n_scen + cl - 1) / cl;
+            const long waves = (ctas + 148 * per_sm - 1) / (148 * per_sm);
+            const long cost = waves * (4 + cl);
+            if (waves > (esz == 4 || per_sm == 1 ? 3 : 2) || (r.cl && cost >= best_cost)) continue;
+            r.cl = cl;
+            r.threads = thr;
+            r.carveout = (int)std::min<long>(
+                100, (100 * std::min(per_sm, (ctas + 147) / 148) * per_cta + SMALL_SM_SMEM - 1) / SMALL_SM_SMEM);
+            best_cost = cost;
+        }
+    }
+    r.together &= r.cl < b->sw;  // one CTA holds the whole group otherwise
+    return r;
+}
+
+template <typename T, int CL>
+struct SmallOp {
+    static void run(gapk_nr_batch b, SmallRun r, int refine, int passes, cudaStream_t st) {
+        auto const& h = b->plan->h;
+        cudaLaunchConfig_t cfg{};
+        // what shared memory the launch does not need is left to L1, which holds the lists
+        cudaLaunchAttribute attr[2]{};
+        attr[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[0].val.sharedMemCarveout = r.carveout;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = b->sw / CL;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(b->G * (b->sw / CL));
+        cfg.blockDim = dim3(r.threads);
+        cfg.dynamicSmemBytes =
+            small_layout(h.n_bus, h.nb, h.n_slots, h.n_tail, h.n_levels, CL, sizeof(T)).total;
+        cfg.stream = st;
+        cfg.attrs = attr;
+        cfg.numAttrs = r.together ? 2 : 1;
+        cudaLaunchKernelEx(&cfg, k_nr_small<T, CL>, b->plan->dev, b->dev, refine, r.together, passes);
+    }
+};
+template <typename T>
+cudaError_t small_attributes() {
+    auto set = [](auto fn) {
+        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_SMEM_MAX);
+    };
+    cudaError_t e = set(k_nr_small<T, 1>);
+    if (e == cudaSuccess) e = set(k_nr_small<T, 2>);
+    if (e == cudaSuccess) e = set(k_nr_small<T, 4>);
+    if (e == cudaSuccess) e = set(k_nr_small<T, 8>);
+    return e;
+}
+
 int load_inputs(gapk_nr_batch b, const gapk_nr_inputs* in, cudaStream_t st) {
-    if (!in || !in->d_y || !in->d_s_spec) {
-        set_error("inputs: d_y and d_s_spec are required");
-        return GAPK_EINVAL;
-    }
-    if (in->max_iterations < 0 || in->refine < 0 || in->refine > 8 ||
-        (in->policy < GAPK_POLICY_REFERENCE || in->policy > GAPK_POLICY_CLAMPED)) {
-        set_error("inputs: bad max_iterations / refine / policy");
-        return GAPK_EINVAL;
-    }
-    if (in->refine > 0 && !b->A64.p) {
-        set_error("inputs: refine > 0 needs a batch created with precision FP32");
-        return GAPK_EINVAL;
-    }
+    int rc = validate_inputs(b, in);
+    if (rc) return rc;
     b->cur_refine = in->refine;
-    // iteration, max iterations, loop flag, step policy, iterations run, device wait error
-    int ctrl[6] = {0, in->max_iterations, 1, in->policy, 0, 0};
-    GAPK_CUDA_TRY(cudaMemcpyAsync(b->ctrl.p, ctrl, sizeof(ctrl), cudaMemcpyHostToDevice, st));
-    if (!(in->refine_below >= 0.0) || !(in->reuse_below >= 0.0)) {
-        set_error("inputs: refine_below and reuse_below must be >= 0");
-        return GAPK_EINVAL;
-    }
-    if (in->reuse_below > 0.0 && in->refine < 1) {
-        set_error("inputs: reuse_below > 0 needs refine >= 1");
-        return GAPK_EINVAL;
-    }
-    double tol[3] = {in->tolerance, in->refine_below, in->reuse_below};
-    GAPK_CUDA_TRY(cudaMemcpyAsync(b->tol.p, tol, sizeof(tol), cudaMemcpyHostToDevice, st));
+    b->cur_small = small_choice(b, in);
     dispatch_tsw<LoadOp>(b->precision, b->sw, b, in, st);
     return check_launch();
 }
@@ -735,6 +885,13 @@ int gapk_nr_batch_create(gapk_nr_plan p, int n_scen, const gapk_nr_batch_options
             return GAPK_ECUDA;
         }
     }
+    if (p->dev.levels) {
+        cudaError_t e = esz == 8 ? small_attributes<double>() : small_attributes<float>();
+        if (e != cudaSuccess) {
+            set_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
+            return GAPK_ECUDA;
+        }
+    }
     A(b->mis, L * 8);
     A(b->state, L * 4);
     A(b->solving, L * 4);
@@ -816,7 +973,11 @@ int gapk_nr_solve(gapk_nr_batch b, const gapk_nr_inputs* in, const gapk_nr_outpu
     int rc = load_inputs(b, in, st);
     if (rc) return rc;
     if (in->max_iterations > 0) {
-        if (b->use_graph) {
+        if (const SmallRun r = b->cur_small; r.cl) {
+            dispatch_tsw<SmallOp>(b->precision, r.cl, b, r, in->refine, 0, st);
+            rc = check_launch();
+            if (rc) return rc;
+        } else if (b->use_graph) {
             rc = build_graph(b, st);
             if (rc) return rc;
             GAPK_CUDA_TRY(cudaGraphLaunch(b->exec, st));
@@ -928,7 +1089,13 @@ int gapk_nr_step(gapk_nr_batch b, int* h_active, void* stream) {
         return GAPK_EINVAL;
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    dispatch_tsw<BodyOp>(b->precision, b->sw, b, st, 0, cudaGraphConditionalHandle{});
+    if (const SmallRun r = b->cur_small; r.cl) {
+        k_small_step<<<1, 256, 0, st>>>(b->dev, 0);
+        dispatch_tsw<SmallOp>(b->precision, r.cl, b, r, b->cur_refine, 1, st);
+        k_small_step<<<1, 256, 0, st>>>(b->dev, 1);
+    } else {
+        dispatch_tsw<BodyOp>(b->precision, b->sw, b, st, 0, cudaGraphConditionalHandle{});
+    }
     int rc = check_launch();
     if (rc) return rc;
     GAPK_CUDA_TRY(cudaMemcpyAsync(h_active, b->dev.ctrl + 2, sizeof(int),
@@ -979,6 +1146,7 @@ int gapk_nr_batch_set_wait_test(gapk_nr_batch b, int skip) {
         return GAPK_EINVAL;
     }
     const int v = skip ? 1 : 0;
+    b->wait_test = v;
     GAPK_CUDA_TRY(cudaMemcpy(b->ctrl.as<int>() + 6, &v, sizeof(int), cudaMemcpyHostToDevice));
     return GAPK_OK;
 }
@@ -1029,18 +1197,11 @@ namespace gapk {
 namespace {
 
 template <typename T, int SW>
-struct InitOp {
-    static void run(gapk_nr_batch b, const gapk_nr_inputs* in, cudaStream_t st) {
-        k_init_ctrl<<<1, 32, 0, st>>>(b->dev, in->max_iterations, in->policy, in->tolerance,
-                                     in->refine_below, in->reuse_below);
-    }
-};
-template <typename T, int SW>
 struct RetryOp {
-    static void run(gapk_nr_batch b, const gapk_nr_inputs* in, int policy,
+    static void run(gapk_nr_batch b, const gapk_nr_inputs* in, int policy, int use_cond,
                     cudaGraphConditionalHandle h, cudaStream_t st) {
         PlanDev const& P = b->plan->dev;
-        k_retry_flags<SW><<<1, 1024, 0, st>>>(b->dev, policy, h);
+        k_retry_flags<SW><<<1, 1024, 0, st>>>(b->dev, policy, use_cond, h);
         dim3 g(blocks_for((long)P.n_bus * SW, 256), b->G);
         k_retry_v<SW><<<g, 256, 0, st>>>(P, b->dev, reinterpret_cast<const double2*>(in->d_v_init),
                                          in->d_u_pu, in->v_init_shared);
@@ -1121,11 +1282,20 @@ struct gapk_nr_mix_s {
                 return GAPK_ECUDA;
             }
             int rc = GAPK_OK;
-            dispatch_tsw<InitOp>(b->precision, b->sw, b, &ins[i], cs);
             dispatch_tsw<LoadOp>(b->precision, b->sw, b, &ins[i], cs);
             cudaGraphConditionalHandle h{};
-            if (ins[i].max_iterations > 0) rc = add_loop(b, cs, body, 1, &h);
-            if (!rc && retry_policy >= 0 && ins[i].max_iterations > 0) {
+            const SmallRun sm = ins[i].max_iterations > 0 ? small_choice(b, &ins[i]) : SmallRun{};
+            if (sm.cl) {
+                // the retry is the same kernel again: groups without a retried scenario return
+                dispatch_tsw<SmallOp>(b->precision, sm.cl, b, sm, ins[i].refine, 0, cs);
+                if (retry_policy >= 0) {
+                    dispatch_tsw<RetryOp>(b->precision, b->sw, b, &ins[i], retry_policy, 0, h, cs);
+                    dispatch_tsw<SmallOp>(b->precision, sm.cl, b, sm, ins[i].refine, 0, cs);
+                }
+            } else if (ins[i].max_iterations > 0) {
+                rc = add_loop(b, cs, body, 1, &h);
+            }
+            if (!rc && !sm.cl && retry_policy >= 0 && ins[i].max_iterations > 0) {
                 cudaGraphConditionalHandle r{};
                 // the retry loop's condition starts false; k_retry_flags sets it
                 rc = add_loop_after(b, &ins[i], retry_policy, &r);
@@ -1155,7 +1325,7 @@ struct gapk_nr_mix_s {
         GAPK_CUDA_TRY(cudaStreamGetCaptureInfo(cs, &stat, nullptr, &g, nullptr, nullptr));
         cudaGraphConditionalHandle r;
         GAPK_CUDA_TRY(cudaGraphConditionalHandleCreate(&r, g, 0, cudaGraphCondAssignDefault));
-        dispatch_tsw<RetryOp>(b->precision, b->sw, b, in, policy, r, cs);
+        dispatch_tsw<RetryOp>(b->precision, b->sw, b, in, policy, 1, r, cs);
         // the while node reads the condition k_retry_flags set
         cudaStreamCaptureStatus stat2;
         const cudaGraphNode_t* deps = nullptr;
@@ -1308,6 +1478,7 @@ int gapk_splu_create(int n, int nnz, const int* h_row_ptr, const int* h_col_idx,
         return GAPK_EINVAL;
     }
     auto s = std::make_unique<gapk_splu_s>();
+    s->plan.general = true;
     try {
         if (!analyze_general(n, nnz, h_row_ptr, h_col_idx, 16, s->plan.h, s->rp, s->val_map))
             return GAPK_EINVAL;
@@ -1456,12 +1627,13 @@ extern "C" int gapk_nr_solve_noalloc(gapk_nr_plan p, const gapk_nr_inputs* in,
     }
     auto const& h = p->h;
     const size_t n = h.n_bus, nb = h.nb, nnz = h.nnz_y, N = 2 * (size_t)h.n_tail;
+    const std::vector<int> a_rec = p->a_records();
     // plan index lists copied into the scratch, in this order
     std::vector<int> const* lists[] = {&p->y_row_ptr, &p->y_col, &h.bus_type, &h.node_of_bus,
-                                       &h.slot_info, &h.slot_src, &h.slot_a, &h.level_ptr,
+                                       &h.slot_info, &h.slot_src, &h.level_ptr,
                                        &h.level_nodes, &h.fa_ptr, &h.targets, &h.pairs,
                                        &h.fb_ptr, &h.scale, &h.lptr, &h.lidx, &h.rptr,
-                                       &h.rlist, &h.arow_ptr, &h.arow, &h.schur, &h.a_slots};
+                                       &h.rlist, &h.schur, &a_rec};
     constexpr int kLists = sizeof(lists) / sizeof(lists[0]);
     Carver c;
     size_t loff[kLists];
@@ -1525,22 +1697,19 @@ extern "C" int gapk_nr_solve_noalloc(gapk_nr_plan p, const gapk_nr_inputs* in,
     P.node_of_bus = L(3);
     P.slot_info = reinterpret_cast<const int4*>(L(4));
     P.slot_src = L(5);
-    P.slot_a = L(6);
-    P.level_ptr = L(7);
-    P.level_nodes = L(8);
-    P.fa_ptr = L(9);
-    P.targets = reinterpret_cast<const int4*>(L(10));
-    P.pairs = reinterpret_cast<const int2*>(L(11));
-    P.fb_ptr = L(12);
-    P.scale = reinterpret_cast<const int2*>(L(13));
-    P.lptr = L(14);
-    P.lidx = L(15);
-    P.rptr = L(16);
-    P.rlist = reinterpret_cast<const int2*>(L(17));
-    P.arow_ptr = L(18);
-    P.arow = reinterpret_cast<const int2*>(L(19));
-    P.schur = reinterpret_cast<const int4*>(L(20));
-    P.a_slots = L(21);
+    P.level_ptr = L(6);
+    P.level_nodes = L(7);
+    P.fa_ptr = L(8);
+    P.targets = reinterpret_cast<const int4*>(L(9));
+    P.pairs = reinterpret_cast<const int2*>(L(10));
+    P.fb_ptr = L(11);
+    P.scale = reinterpret_cast<const int2*>(L(12));
+    P.lptr = L(13);
+    P.lidx = L(14);
+    P.rptr = L(15);
+    P.rlist = reinterpret_cast<const int2*>(L(16));
+    P.schur = reinterpret_cast<const int4*>(L(17));
+    P.a_rec = reinterpret_cast<const int4*>(L(18));
     BatchDev D{};
     D.n_scen = 1;
     D.n_groups = 1;
@@ -1576,7 +1745,7 @@ extern "C" int gapk_nr_solve_noalloc(gapk_nr_plan p, const gapk_nr_inputs* in,
     k_load<1><<<blocks_for((long)n, 256), 256, 0, st>>>(
         P, D, reinterpret_cast<const double2*>(in->d_y),
         reinterpret_cast<const double2*>(in->d_s_spec),
-        reinterpret_cast<const double2*>(in->d_v_init), in->d_u_pu, 0);
+        reinterpret_cast<const double2*>(in->d_v_init), in->d_u_pu, 0, SolveOpts{});
     rc = check_launch();
     if (rc) return rc;
     const int thr = 512;

@@ -27,6 +27,7 @@ struct PlanDev {
     int ns, n_tail, n_schur;  // sparse nodes, dense-tail nodes, Schur targets (= n_tail^2)
     const int4* schur;        // (slot, pair_begin, pair_end, position r*n_tail+c | hasval<<30)
     const int* a_slots;       // slots holding Jacobian values (the only ones the fill writes)
+    const int4* a_rec;        // per Jacobian block: slot, row bus, column bus, Y entry (jac_block)
     const int* acol_ptr;      // A blocks by block column: (a index, row node)
     const int2* acol;
     const int* y_row_ptr;
@@ -35,9 +36,11 @@ struct PlanDev {
     const int* node_of_bus;
     const int4* slot_info;
     const int* slot_src;
-    const int* slot_a;
     const int* level_ptr;
     const int* level_nodes;
+    const int4* levels;       // k_nr_small's level records and packed schedule (null when the
+    const unsigned* words;    // grid is too large for it)
+    const uint2* ell;
     const int* fa_ptr;
     const int4* targets;
     const int2* pairs;
@@ -105,15 +108,33 @@ __device__ __forceinline__ void lvl_stamp(BatchDev const& B, int n_levels, int w
 // ---------------------------------------------------------------------------------------
 // load: interleave inputs, flat start, reset state
 // ---------------------------------------------------------------------------------------
+// Loop options of one solve, kernel arguments of k_load (no host copies, so that a graph can hold
+// several batches' solves); set = 0 leaves the control words and tolerances to the caller.
+struct SolveOpts {
+    int set, max_iter, policy;
+    double tol, refine_below, reuse_below;
+};
+
 template <int SW>
 __global__ void k_load(PlanDev P, BatchDev B, const double2* __restrict__ y_in,
                        const double2* __restrict__ s_in, const double2* __restrict__ v_in,
-                       const double* __restrict__ u_pu, int v_shared) {
+                       const double* __restrict__ u_pu, int v_shared, SolveOpts opt) {
     const int g = blockIdx.y;
     const int n = P.n_bus;
     const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int i = (int)(tid / SW), lane = (int)(tid % SW);
     int q = g * SW + lane;
+    if (opt.set && g == 0 && tid == 0) {
+        B.ctrl[0] = 0;
+        B.ctrl[1] = opt.max_iter;
+        B.ctrl[2] = 1;
+        B.ctrl[3] = opt.policy;
+        B.ctrl[4] = 0;
+        B.ctrl[5] = 0;  // set by a tensor-core LU whose bounded wait ran out during the solve
+        B.tol[0] = opt.tol;
+        B.tol[1] = opt.refine_below;
+        B.tol[2] = opt.reuse_below;
+    }
     int src = q < B.n_scen ? q : g * SW;  // padding lanes mirror the group's first scenario
     if (i < n) {
         size_t o = ((size_t)g * n + i) * SW + lane;
@@ -155,31 +176,14 @@ __global__ void k_load(PlanDev P, BatchDev B, const double2* __restrict__ y_in,
 }
 
 // ---------------------------------------------------------------------------------------
-// in-graph control: solve options as kernel arguments, and the retry of unconverged lanes
+// in-graph control: the retry of unconverged lanes
 // ---------------------------------------------------------------------------------------
-// Loop control words and tolerances of one solve, written on the device (a graph that holds
-// several batches' loops sets each batch's options without host copies).
-__global__ void k_init_ctrl(BatchDev B, int max_iter, int policy, double tol, double refine_below,
-                            double reuse_below) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        B.ctrl[0] = 0;
-        B.ctrl[1] = max_iter;
-        B.ctrl[2] = 1;
-        B.ctrl[3] = policy;
-        B.ctrl[4] = 0;
-        B.ctrl[5] = 0;  // set by a tensor-core LU whose bounded wait ran out during the solve
-        B.tol[0] = tol;
-        B.tol[1] = refine_below;
-        B.tol[2] = reuse_below;
-    }
-}
-
 // Retry after the loop (one CTA): every scenario that ended at max_iterations or with a
 // non-finite mismatch starts again with the step policy `policy` (its other scenarios stay
-// done); the groups holding one iterate again, refactorising and refining.  Sets the retry
-// loop's condition to whether any scenario retries.
+// done); the groups holding one iterate again, refactorising and refining.  With use_cond, sets
+// the retry loop's condition to whether any scenario retries.
 template <int SW>
-__global__ void k_retry_flags(BatchDev B, int policy, cudaGraphConditionalHandle handle) {
+__global__ void k_retry_flags(BatchDev B, int policy, int use_cond, cudaGraphConditionalHandle handle) {
     __shared__ int any;
     if (threadIdx.x == 0) any = 0;
     __syncthreads();
@@ -213,7 +217,7 @@ __global__ void k_retry_flags(BatchDev B, int policy, cudaGraphConditionalHandle
         B.ctrl[0] = 0;
         B.ctrl[2] = any;
         B.ctrl[3] = policy;
-        cudaGraphSetConditional(handle, any ? 1u : 0u);
+        if (use_cond) cudaGraphSetConditional(handle, any ? 1u : 0u);
     }
 }
 
@@ -427,6 +431,83 @@ __device__ __forceinline__ void polar_parts(double2 v, double& vmr, double& c, d
     vmr = vm < 1e-6 ? 1.0 : vm;
 }
 
+// The Jacobian block of bus i's own entry (G + jB its diagonal admittance, S its power).
+__device__ __forceinline__ Blk<double> jac_diag(double G, double Bv, double2 v, double2 S, bool pq) {
+    double n = v.x * v.x + v.y * v.y, ivm = rsqrt(n), vm = n * ivm;
+    if (n < 1.1e-12) {  // |V| below 1e-6 counts as 1
+        double c, s;
+        polar_parts(v, vm, c, s);
+        n = vm * vm;
+        ivm = 1.0 / vm;
+    }
+    if (!pq) return {-S.y - Bv * n, 0.0, 0.0, 1.0};
+    return {-S.y - Bv * n, S.x * ivm + G * vm, S.x - G * n, S.y * ivm - Bv * vm};
+}
+// The block of buses i (row) and j (column) joined by the admittance G + jB: with the products
+// |V_i||V_j| cos / sin(theta_i - theta_j) = Re / Im(V_i conj(V_j)) it needs one reciprocal root
+// and no polar form (two hypot and two divisions made the fill FP64-issue bound).
+__device__ __forceinline__ Blk<double> jac_off(double G, double Bv, double2 vi, double2 vj, bool pqi,
+                                               bool pqj) {
+    const double ni = vi.x * vi.x + vi.y * vi.y, nj = vj.x * vj.x + vj.y * vj.y;
+    double pr = vi.x * vj.x + vi.y * vj.y, pi = vi.y * vj.x - vi.x * vj.y, rj = rsqrt(nj);
+    if (ni < 1.1e-12 || nj < 1.1e-12) {  // |V| below 1e-6 counts as 1, along its direction
+        double vmi, ci, sni, vmj, cj, snj;
+        polar_parts(vi, vmi, ci, sni);
+        polar_parts(vj, vmj, cj, snj);
+        pr = vmi * vmj * (ci * cj + sni * snj);
+        pi = vmi * vmj * (sni * cj - ci * snj);
+        rj = 1.0 / vmj;
+    }
+    const double t = G * pr + Bv * pi, u = G * pi - Bv * pr;
+    Blk<double> J = {u, t * rj, -t, u * rj};
+    if (!pqi) {
+        J.c = 0.0;
+        J.d = 0.0;
+    }
+    if (!pqj) {
+        J.b = 0.0;
+        J.d = 0.0;
+    }
+    return J;
+}
+// Reference mode: convert_to_sparse_matrix drops |x| <= 1e-12 (cpu_newton_raphson.cpp:754).
+__device__ __forceinline__ void jac_drop(Blk<double>& J, bool diag) {
+    if (fabs(J.a) <= 1e-12) J.a = 0.0;
+    if (fabs(J.b) <= 1e-12) J.b = 0.0;
+    if (fabs(J.c) <= 1e-12) J.c = 0.0;
+    if (fabs(J.d) <= 1e-12 && !(diag && J.d == 1.0)) J.d = 0.0;
+}
+
+// One record per Jacobian block (P.a_rec): its slot, its row and column bus (bit 30: a PQ bus)
+// and the Y entry it is made of, or -1 where the sources are listed (none, or several) -- one
+// load where slot, slot_info, slot_src and the bus types were a chain of four.
+constexpr int REC_PQ = 1 << 30, REC_BUS = REC_PQ - 1;
+
+// Block a of the Jacobian at voltages v(bus), powers s(bus) and admittances y(entry).
+template <typename FV, typename FS, typename FY>
+__device__ __forceinline__ Blk<double> jac_block(PlanDev const& P, int4 rec, FV v, FS s, FY y) {
+    const int i = rec.y & REC_BUS, j = rec.z & REC_BUS;
+    const bool diag = i == j, pqi = rec.y & REC_PQ, pqj = rec.z & REC_PQ;
+    const double2 vi = v(i), vj = v(j);
+    double G = 0.0, Bv = 0.0;
+    if (rec.w >= 0) {
+        const double2 a = y(rec.w);
+        G = a.x;
+        Bv = a.y;
+    } else {
+        const int4 si = P.slot_info[rec.x];
+        if (!diag && si.z >= si.w) return {0.0, 0.0, 0.0, 0.0};
+        for (int e = si.z; e < si.w; ++e) {
+            const double2 a = y(P.slot_src[e]);
+            G += a.x;
+            Bv += a.y;
+        }
+    }
+    Blk<double> J = diag ? jac_diag(G, Bv, vi, s(i), pqi) : jac_off(G, Bv, vi, vj, pqi, pqj);
+    if (P.jac_mode == 0) jac_drop(J, diag);
+    return J;
+}
+
 template <typename T, int SW>
 __global__ void __launch_bounds__(256) k_jfill(PlanDev P, BatchDev B) {
     const int g = blockIdx.y;
@@ -434,66 +515,12 @@ __global__ void __launch_bounds__(256) k_jfill(PlanDev P, BatchDev B) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int a_idx = tid / SW, lane = tid % SW;
     if (a_idx >= P.n_a) return;
-    const int slot = P.a_slots[a_idx];
-    const int4 si = P.slot_info[slot];
-    const int n = P.n_bus;
-    Blk<double> J = {0.0, 0.0, 0.0, 0.0};
-    const bool diag = si.x == si.y;
-    if (diag || si.z < si.w) {
-        double G = 0.0, Bv = 0.0;
-#pragma unroll 4
-        for (int e = si.z; e < si.w; ++e) {
-            const int p = P.slot_src[e];
-            const double2 y = B.y_shared ? B.Y[p] : B.Y[((size_t)g * P.nnz_y + p) * SW + lane];
-            G += y.x;
-            Bv += y.y;
-        }
-        const double2* Vg = B.V + (size_t)g * n * SW;
-        const bool pqi = P.bus_type[si.x] == BUS_PQ;
-        double vmi, ci, sni;
-        polar_parts(Vg[(size_t)si.x * SW + lane], vmi, ci, sni);
-        if (diag) {
-            const double2 S = B.Scalc[((size_t)g * n + si.x) * SW + lane];
-            J.a = -S.y - Bv * vmi * vmi;
-            const double ivm = 1.0 / vmi;
-            J.b = S.x * ivm + G * vmi;
-            J.c = S.x - G * vmi * vmi;
-            J.d = S.y * ivm - Bv * vmi;
-            if (!pqi) {
-                J.b = 0.0;
-                J.c = 0.0;
-                J.d = 1.0;
-            }
-        } else {
-            const bool pqj = P.bus_type[si.y] == BUS_PQ;
-            double vmj, cj, snj;
-            polar_parts(Vg[(size_t)si.y * SW + lane], vmj, cj, snj);
-            // u = |V_i| e^{j(theta_i - theta_j)}
-            const double uc = vmi * (ci * cj + sni * snj);
-            const double ud = vmi * (sni * cj - ci * snj);
-            const double gcbd = G * uc + Bv * ud;
-            const double gdbc = G * ud - Bv * uc;
-            J.a = vmj * gdbc;
-            J.b = gcbd;
-            J.c = -vmj * gcbd;
-            J.d = gdbc;
-            if (!pqi) {
-                J.c = 0.0;
-                J.d = 0.0;
-            }
-            if (!pqj) {
-                J.b = 0.0;
-                J.d = 0.0;
-            }
-        }
-    }
-    if (P.jac_mode == 0) {
-        // convert_to_sparse_matrix drops |x| <= 1e-12 (cpu_newton_raphson.cpp:754)
-        if (fabs(J.a) <= 1e-12) J.a = 0.0;
-        if (fabs(J.b) <= 1e-12) J.b = 0.0;
-        if (fabs(J.c) <= 1e-12) J.c = 0.0;
-        if (fabs(J.d) <= 1e-12 && !(diag && J.d == 1.0)) J.d = 0.0;
-    }
+    const int4 rec = P.a_rec[a_idx];
+    const int slot = rec.x, n = P.n_bus;
+    const Blk<double> J = jac_block(
+        P, rec, [&](int i) { return B.V[((size_t)g * n + i) * SW + lane]; },
+        [&](int i) { return B.Scalc[((size_t)g * n + i) * SW + lane]; },
+        [&](int p) { return B.y_shared ? B.Y[p] : B.Y[((size_t)g * P.nnz_y + p) * SW + lane]; });
     if (!B.gfactor || B.gfactor[g]) {  // a group that reuses its factors keeps them
         Blk<T>* F = reinterpret_cast<Blk<T>*>(B.F) + ((size_t)g * P.n_slots + slot) * SW + lane;
         stb(F, Blk<T>{(T)J.a, (T)J.b, (T)J.c, (T)J.d});
@@ -1492,41 +1519,12 @@ __global__ void __launch_bounds__(256, 8) k_residual(PlanDev P, BatchDev B) {
 // ---------------------------------------------------------------------------------------
 // voltage update
 // ---------------------------------------------------------------------------------------
-template <int SW>
-__global__ void __launch_bounds__(256, 8) k_update(PlanDev P, BatchDev B) {
-    const int g = blockIdx.y;
-    if (!B.gsolve[g]) return;
-    const int n = P.n_bus;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = tid / SW, lane = tid % SW;
-    if (i >= n) return;
-    const int q = g * SW + lane;
-    // the loads that do not depend on the flags below go first (padding lanes have storage),
-    // so that one memory latency covers them and the flags
-    const int node = P.node_of_bus[i];
-    const size_t o = ((size_t)g * n + i) * SW + lane;
-    double2 v = B.V[o];
-    const bool pq = P.bus_type[i] == BUS_PQ;
-    const double2 d = node >= 0 ? B.dx[((size_t)g * P.nb + node) * SW + lane] : make_double2(0.0, 0.0);
-    if (q >= B.n_scen) return;  // padding lanes are never updated
-    {
-        if (B.singular[q]) {
-            // the reference keeps V unchanged when factorize() fails and runs to max_iter
-            if (i == 0 && B.solving[q]) {
-                B.state[q] = 1;
-                B.status[q] = SC_SINGULAR;
-                B.iters[q] = B.ctrl[1];
-                B.solving[q] = 0;
-            }
-            return;
-        }
-        if (!B.solving[q]) return;
-    }
-    if (node < 0) return;
-    if (B.ctrl[3] != 1) {
+// One bus's voltage after the Newton correction d = (dtheta, d|V|), by step policy.
+__device__ __forceinline__ double2 newton_step(double2 v, double2 d, bool pq, int policy) {
+    if (policy != 1) {
         // reference policy (cpu_newton_raphson.cpp:457-503): damping 0.9 and the clamps;
         // clamped policy: the same clamps and order with the full step
-        const double damp = B.ctrl[3] == 0 ? 0.9 : 1.0;
+        const double damp = policy == 0 ? 0.9 : 1.0;
         const double vm = hypot(v.x, v.y);
         double a = damp * d.x;
         if (fabs(a) > 0.15) a = 0.15 * (a > 0 ? 1.0 : -1.0);
@@ -1558,7 +1556,41 @@ __global__ void __launch_bounds__(256, 8) k_update(PlanDev P, BatchDev B) {
             v = make_double2(m * cs, m * sn);
         }
     }
-    B.V[o] = v;
+    return v;
+}
+
+template <int SW>
+__global__ void __launch_bounds__(256, 8) k_update(PlanDev P, BatchDev B) {
+    const int g = blockIdx.y;
+    if (!B.gsolve[g]) return;
+    const int n = P.n_bus;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = tid / SW, lane = tid % SW;
+    if (i >= n) return;
+    const int q = g * SW + lane;
+    // the loads that do not depend on the flags below go first (padding lanes have storage),
+    // so that one memory latency covers them and the flags
+    const int node = P.node_of_bus[i];
+    const size_t o = ((size_t)g * n + i) * SW + lane;
+    double2 v = B.V[o];
+    const bool pq = P.bus_type[i] == BUS_PQ;
+    const double2 d = node >= 0 ? B.dx[((size_t)g * P.nb + node) * SW + lane] : make_double2(0.0, 0.0);
+    if (q >= B.n_scen) return;  // padding lanes are never updated
+    {
+        if (B.singular[q]) {
+            // the reference keeps V unchanged when factorize() fails and runs to max_iter
+            if (i == 0 && B.solving[q]) {
+                B.state[q] = 1;
+                B.status[q] = SC_SINGULAR;
+                B.iters[q] = B.ctrl[1];
+                B.solving[q] = 0;
+            }
+            return;
+        }
+        if (!B.solving[q]) return;
+    }
+    if (node < 0) return;
+    B.V[o] = newton_step(v, d, pq, B.ctrl[3]);
 }
 
 // ---------------------------------------------------------------------------------------
