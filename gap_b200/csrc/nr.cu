@@ -75,7 +75,7 @@ struct gapk_nr_plan_s {
     // device copy (current device at first upload)
     bool uploaded = false;
     int device = -1;
-    DevBuf d_yrp, d_ycol, d_bt, d_nob, d_si, d_ss, d_lp, d_ln, d_fa, d_tg, d_pr, d_fb,
+    DevBuf d_yrp, d_ycol, d_bt, d_nob, d_si, d_ss, d_lp, d_fa, d_tg, d_pr, d_fb,
         d_sc, d_lptr, d_lidx, d_rptr, d_rl, d_arp, d_ar, d_var, d_eq, d_schur, d_aslots, d_arec, d_levels, d_words, d_ell, d_acp, d_ac;
     PlanDev dev{};
 
@@ -174,7 +174,6 @@ struct gapk_nr_plan_s {
         up(d_si, h.slot_info);
         up(d_ss, h.slot_src);
         up(d_lp, h.level_ptr);
-        up(d_ln, h.level_nodes);
         up(d_fa, h.fa_ptr);
         up(d_tg, h.targets);
         up(d_pr, h.pairs);
@@ -228,7 +227,6 @@ struct gapk_nr_plan_s {
         dev.slot_info = d_si.as<int4>();
         dev.slot_src = d_ss.as<int>();
         dev.level_ptr = d_lp.as<int>();
-        dev.level_nodes = d_ln.as<int>();
         dev.fa_ptr = d_fa.as<int>();
         dev.targets = d_tg.as<int4>();
         dev.pairs = d_pr.as<int2>();
@@ -253,6 +251,8 @@ struct gapk_nr_batch_s {
     gapk_nr_plan plan = nullptr;
     int n_scen = 0, sw = 8, G = 0, precision = 0, y_shared = 1, threads = 256, use_graph = 1;
     int dense_fused = 0;
+    int level_ctas = 1;  // CTAs per lane group of the level-scheduled kernels
+    int split_slots = 0; // k_factor's split_slots
     DevBuf V, Sspec, Scalc, Y, F, A64, rhs, dx, res, X, Dt, mis, state, solving, singular,
         iters, status, fmis, gsolve, giter, grefine, gfactor, ctrl, tol;
     int dense_w = 0;          // panel width of the one-CTA-per-scenario dense LU (0: not used)
@@ -279,21 +279,37 @@ inline unsigned blocks_for(long items, int threads) {
     return static_cast<unsigned>((items + threads - 1) / threads);
 }
 
+// A level-scheduled kernel, b->level_ctas CTAs (one cluster) per lane group.
+template <typename K, typename... A>
+void launch_levels(gapk_nr_batch b, cudaStream_t st, K kernel, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute cluster{};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = b->level_ctas;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(b->G * b->level_ctas);
+    cfg.blockDim = dim3(b->threads);
+    cfg.stream = st;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = b->level_ctas > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <typename T, int SW>
 void launch_solve(gapk_nr_batch b, cudaStream_t st, const double2* rhs, double2* out, int acc) {
     PlanDev const& P = b->plan->dev;
     BatchDev const& B = b->dev;
-    k_solve_fwd<T, SW><<<b->G, b->threads, 0, st>>>(P, B, rhs, acc);
+    launch_levels(b, st, k_solve_fwd<T, SW, false>, P, B, rhs, acc);
     if (P.n_tail > 0)
         k_dense_solve<T, SW><<<b->G * SW, 256, dense_solve_smem(P.n_tail, sizeof(T)), st>>>(P, B, out, acc);
-    k_solve_bwd<T, SW><<<b->G, b->threads, 0, st>>>(P, B, out, acc);
+    launch_levels(b, st, k_solve_bwd<T, SW, false>, P, B, out, acc);
 }
 
 template <typename T, int SW>
 void launch_factor(gapk_nr_batch b, cudaStream_t st) {
     PlanDev const& P = b->plan->dev;
     BatchDev const& B = b->dev;
-    k_factor<T, SW><<<b->G, b->threads, 0, st>>>(P, B);
+    launch_levels(b, st, k_factor<T, SW>, P, B, b->split_slots);
     if (P.n_tail > 0) {
         dim3 gs(blocks_for((long)P.n_schur * SW, 256), b->G);
         k_schur<T, SW><<<gs, 256, 0, st>>>(P, B);
@@ -429,7 +445,7 @@ struct KernelOp {
         switch (which) {
             case 0: k_mismatch<SW><<<mismatch_grid<SW>(P, G), 256, 0, st>>>(P, B); break;
             case 1: k_jfill<T, SW><<<dim3(blocks_for((long)P.n_a * SW, 256), G), 256, 0, st>>>(P, B); break;
-            case 2: k_factor<T, SW><<<G, b->threads, 0, st>>>(P, B); break;
+            case 2: launch_levels(b, st, k_factor<T, SW>, P, B, b->split_slots); break;
             case 3:
                 if (P.n_tail > 0)
                     k_schur<T, SW><<<dim3(blocks_for((long)P.n_schur * SW, 256), G), 256, 0, st>>>(P, B);
@@ -441,12 +457,12 @@ struct KernelOp {
                     else
                         launch_dense_lu<T>(b->dense_w, G * SW, b->dense_smem, st, B, 2 * P.n_tail, b->dense_tc);
                 break;
-            case 5: k_solve_fwd<T, SW><<<G, b->threads, 0, st>>>(P, B, B.rhs, 0); break;
+            case 5: launch_levels(b, st, k_solve_fwd<T, SW, false>, P, B, (const double2*)B.rhs, 0); break;
             case 6:
                 if (P.n_tail > 0)
                     k_dense_solve<T, SW><<<G * SW, 256, dense_solve_smem(P.n_tail, sizeof(T)), st>>>(P, B, B.dx, 0);
                 break;
-            case 7: k_solve_bwd<T, SW><<<G, b->threads, 0, st>>>(P, B, B.dx, 0); break;
+            case 7: launch_levels(b, st, k_solve_bwd<T, SW, false>, P, B, B.dx, 0); break;
             case 8: k_update<SW><<<dim3(blocks_for((long)P.n_bus * SW, 256), G), 256, 0, st>>>(P, B); break;
             case 9:
                 if (B.A64) k_residual<SW><<<dim3(blocks_for((long)P.nb * SW, 256), G), 256, 0, st>>>(P, B);
@@ -458,10 +474,10 @@ template <typename T, int SW>
 void launch_solve_t(gapk_nr_batch b, cudaStream_t st, const double2* rhs, double2* out, int acc) {
     PlanDev const& P = b->plan->dev;
     BatchDev const& B = b->dev;
-    k_solve_fwd_t<T, SW><<<b->G, b->threads, 0, st>>>(P, B, rhs);
+    launch_levels(b, st, k_solve_fwd<T, SW, true>, P, B, rhs, 0);
     if (P.n_tail > 0)
         k_dense_solve_t<T, SW><<<b->G * SW, 256, 2 * P.n_tail * sizeof(T), st>>>(P, B, out, acc);
-    k_solve_bwd_t<T, SW><<<b->G, b->threads, 0, st>>>(P, B, out, acc);
+    launch_levels(b, st, k_solve_bwd<T, SW, true>, P, B, out, acc);
 }
 
 template <typename T, int SW>
@@ -513,6 +529,24 @@ struct StateOp {
         k_state<SW><<<blocks_for(total, 256), 256, 0, st>>>(b->plan->dev, b->dev, v, i, s);
     }
 };
+
+// CTA size of the level-scheduled kernels where the caller leaves it open: a thread for every
+// eighth (node, lane), which takes all but the widest levels in one round.  3,001 buses x 333
+// scenarios (42 groups): 8.0 ms with 256 threads, 4.6 ms with 1024.
+int default_threads(int nb, int lanes) {
+    int thr = 256;
+    while (thr < 1024 && 8L * thr < (long)nb * lanes) thr *= 2;
+    return thr;
+}
+// CTAs per lane group of the level-scheduled kernels: as many (a power of two, at most 8) as the
+// 148 SMs hold side by side with all `groups` running.  A batch that shares the GPU with
+// concurrent ones (dense_fused) takes two at most: four parts of 16 groups each took 26.5, 26.0,
+// 28.6 and 37.2 ms with 1, 2, 4 and 8.
+int level_ctas(int groups, int dense_fused) {
+    int nc = 1;
+    while (2 * nc <= (dense_fused ? 2 : 8) && groups * 2 * nc <= 148) nc *= 2;
+    return nc;
+}
 
 int check_launch() {
     cudaError_t e = cudaGetLastError();
@@ -817,7 +851,7 @@ int gapk_nr_batch_create(gapk_nr_plan p, int n_scen, const gapk_nr_batch_options
     }
     b->sw = lanes;
     int thr = opt ? opt->threads : 0;
-    if (thr == 0) thr = lanes == 1 ? 512 : 256;
+    if (thr == 0) thr = default_threads(p->h.nb, lanes);
     if (thr < 32 || thr > 1024 || thr % 32) {
         set_error("gapk_nr_batch_create: threads must be a multiple of 32 in [32, 1024]");
         return GAPK_EINVAL;
@@ -830,6 +864,8 @@ int gapk_nr_batch_create(gapk_nr_plan p, int n_scen, const gapk_nr_batch_options
     auto const& h = p->h;
     const size_t G = (n_scen + lanes - 1) / lanes;
     b->G = static_cast<int>(G);
+    b->level_ctas = level_ctas(b->G, b->dense_fused);
+    b->split_slots = b->level_ctas >= 4 ? b->level_ctas * b->threads / lanes : 0;
     const size_t L = G * lanes;
     const size_t esz = b->precision == GAPK_PREC_FP64 ? 8 : 4;
     const size_t n = h.n_bus, nb = h.nb;
@@ -1272,8 +1308,18 @@ struct gapk_nr_mix_s {
         if (!cs) GAPK_CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
         if (!body) GAPK_CUDA_TRY(cudaStreamCreateWithFlags(&body, cudaStreamNonBlocking));
         GAPK_CUDA_TRY(cudaGraphCreate(&graph, 0));
+        // the branches run side by side: their groups share the SMs (ten studies of 48 groups:
+        // 5.3 ms with the clusters each would have alone, 4.5 ms with two CTAs)
+        int groups = 0;
+        for (gapk_nr_batch b : batches) groups += b->G;
         for (size_t i = 0; i < batches.size(); ++i) {
             gapk_nr_batch b = batches[i];
+            struct Shared {
+                gapk_nr_batch b;
+                int alone;
+                ~Shared() { b->level_ctas = alone; }
+            } shared{b, b->level_ctas};
+            b->level_ctas = std::min(b->level_ctas, level_ctas(groups, 0));
             b->cur_refine = ins[i].refine;
             cudaError_t e = cudaStreamBeginCaptureToGraph(cs, graph, nullptr, nullptr, 0,
                                                           cudaStreamCaptureModeThreadLocal);
@@ -1631,7 +1677,7 @@ extern "C" int gapk_nr_solve_noalloc(gapk_nr_plan p, const gapk_nr_inputs* in,
     // plan index lists copied into the scratch, in this order
     std::vector<int> const* lists[] = {&p->y_row_ptr, &p->y_col, &h.bus_type, &h.node_of_bus,
                                        &h.slot_info, &h.slot_src, &h.level_ptr,
-                                       &h.level_nodes, &h.fa_ptr, &h.targets, &h.pairs,
+                                       &h.fa_ptr, &h.targets, &h.pairs,
                                        &h.fb_ptr, &h.scale, &h.lptr, &h.lidx, &h.rptr,
                                        &h.rlist, &h.schur, &a_rec};
     constexpr int kLists = sizeof(lists) / sizeof(lists[0]);
@@ -1698,18 +1744,17 @@ extern "C" int gapk_nr_solve_noalloc(gapk_nr_plan p, const gapk_nr_inputs* in,
     P.slot_info = reinterpret_cast<const int4*>(L(4));
     P.slot_src = L(5);
     P.level_ptr = L(6);
-    P.level_nodes = L(7);
-    P.fa_ptr = L(8);
-    P.targets = reinterpret_cast<const int4*>(L(9));
-    P.pairs = reinterpret_cast<const int2*>(L(10));
-    P.fb_ptr = L(11);
-    P.scale = reinterpret_cast<const int2*>(L(12));
-    P.lptr = L(13);
-    P.lidx = L(14);
-    P.rptr = L(15);
-    P.rlist = reinterpret_cast<const int2*>(L(16));
-    P.schur = reinterpret_cast<const int4*>(L(17));
-    P.a_rec = reinterpret_cast<const int4*>(L(18));
+    P.fa_ptr = L(7);
+    P.targets = reinterpret_cast<const int4*>(L(8));
+    P.pairs = reinterpret_cast<const int2*>(L(9));
+    P.fb_ptr = L(10);
+    P.scale = reinterpret_cast<const int2*>(L(11));
+    P.lptr = L(12);
+    P.lidx = L(13);
+    P.rptr = L(14);
+    P.rlist = reinterpret_cast<const int2*>(L(15));
+    P.schur = reinterpret_cast<const int4*>(L(16));
+    P.a_rec = reinterpret_cast<const int4*>(L(17));
     BatchDev D{};
     D.n_scen = 1;
     D.n_groups = 1;
@@ -1753,15 +1798,15 @@ extern "C" int gapk_nr_solve_noalloc(gapk_nr_plan p, const gapk_nr_inputs* in,
         k_mismatch<1><<<mismatch_grid<1>(P, 1), 256, 0, st>>>(P, D);
         k_check<1><<<1, 1024, 0, st>>>(D, 0, cudaGraphConditionalHandle{});
         k_jfill<double, 1><<<blocks_for((long)h.n_a, 256), 256, 0, st>>>(P, D);
-        k_factor<double, 1><<<1, thr, 0, st>>>(P, D);
+        k_factor<double, 1><<<1, thr, 0, st>>>(P, D, 0);
         if (h.n_tail > 0) {
             k_schur<double, 1><<<blocks_for((long)P.n_schur, 256), 256, 0, st>>>(P, D);
             launch_dense_lu<double>(dense_w, 1, dense_smem, st, D, (int)N, false);
         }
-        k_solve_fwd<double, 1><<<1, thr, 0, st>>>(P, D, D.rhs, 0);
+        k_solve_fwd<double, 1, false><<<1, thr, 0, st>>>(P, D, D.rhs, 0);
         if (h.n_tail > 0)
             k_dense_solve<double, 1><<<1, 256, dense_solve_smem(P.n_tail, sizeof(double)), st>>>(P, D, D.dx, 0);
-        k_solve_bwd<double, 1><<<1, thr, 0, st>>>(P, D, D.dx, 0);
+        k_solve_bwd<double, 1, false><<<1, thr, 0, st>>>(P, D, D.dx, 0);
         k_update<1><<<blocks_for((long)n, 256), 256, 0, st>>>(P, D);
         rc = check_launch();
         if (rc) return rc;

@@ -37,7 +37,6 @@ struct PlanDev {
     const int4* slot_info;
     const int* slot_src;
     const int* level_ptr;
-    const int* level_nodes;
     const int4* levels;       // k_nr_small's level records and packed schedule (null when the
     const unsigned* words;    // grid is too large for it)
     const uint2* ell;
@@ -98,10 +97,10 @@ __device__ __forceinline__ unsigned long long gtimer() {
     return t;
 }
 // stamp j of kernel `which` for group g: 0 = start, 1 + h = level h done (in execution order),
-// n_levels + 1 = end; one thread per CTA, after a barrier
-__device__ __forceinline__ void lvl_stamp(BatchDev const& B, int n_levels, int which, int g,
-                                          int j) {
-    if (threadIdx.x == 0)
+// n_levels + 1 = end; one thread per group, after a barrier
+__device__ __forceinline__ void lvl_stamp(BatchDev const& B, int n_levels, int which, int g, int j,
+                                          int rank) {
+    if (threadIdx.x == 0 && rank == 0)
         B.lvl_ts[((size_t)which * B.n_groups + g) * (n_levels + 2) + j] = gtimer();
 }
 
@@ -535,22 +534,133 @@ __global__ void __launch_bounds__(256) k_jfill(PlanDev P, BatchDev B) {
 }
 
 // ---------------------------------------------------------------------------------------
-// numeric block LU (left-looking Crout), one CTA per group, level by level
+// The level-scheduled kernels (k_factor, k_solve_fwd, k_solve_bwd) give a lane group one CTA, or
+// a cluster of up to 8 CTAs when the batch has too few groups to fill the GPU (level_ctas): its
+// wide levels are spread over the cluster's threads, with a cluster barrier (release / acquire,
+// so that the other CTAs' global writes are seen) where one CTA has __syncthreads.  How sums are
+// split over threads does not depend on the cluster: the solves split by the CTA size, the
+// factorisation by split_slots, the slots that the batch has when it runs alone (0: no splits).
+// Both are bound by the latency of dependent gathers, level after level.  30,000 buses x 8
+// scenarios (one group, FP32): factor 1,480 -> 363 us, forward 351 -> 130, backward 369 -> 177;
+// 10,000 buses x 256 in FP64 (32 groups, 256 -> 1024 threads a CTA): 2,249 -> 541, 948 -> 209,
+// 954 -> 232 us, of which the CTA size alone 1,041, 335 and 348.
+// ---------------------------------------------------------------------------------------
+struct LevelCta {
+    int nc, rank, g;
+    __device__ __forceinline__ LevelCta() {
+        asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(nc));
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        g = blockIdx.x / nc;
+    }
+    __device__ __forceinline__ void sync() const {
+        if (nc == 1) {
+            __syncthreads();
+        } else {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
+    }
+    // after a level that only rank 0 works on, before another one: the other ranks run ahead
+    __device__ __forceinline__ void sync_solo() const {
+        if (rank == 0) __syncthreads();
+    }
+};
+// Level bounds in shared memory (read once per level by every thread of every CTA).
+constexpr int LV_MAX = 256;
+__device__ __forceinline__ const int* level_bounds(const int* ptr, int n_levels, int* buf) {
+    if (n_levels > LV_MAX) return ptr;
+    for (int i = threadIdx.x; i <= n_levels; i += blockDim.x) buf[i] = ptr[i];
+    return buf;
+}
+
+// Levels with few nodes split every row over s sub-slots (s a power of two, up to 32): the
+// sub-slots of one warp reduce with shuffles, the warps of one row through shared memory.
+// split_factor: the largest s <= 32 with c * s <= ne (at least 1).
+__device__ __forceinline__ int split_factor(int c, int ne) {
+    int s = 1;
+    while (s < 32 && c * s * 2 <= ne) s *= 2;
+    return s;
+}
+
+// Sum `acc` over the s sub-slots of each row (slot e0 = row * s + sub); the result is valid in
+// sub-slot 0.  Every thread of the block calls this (uniform s).
+template <typename T, int SW>
+__device__ __forceinline__ Vec2<T> split_reduce(Vec2<T> acc, int s, int sub, int row, int lane,
+                                                Vec2<T>* red) {
+    constexpr int S = 32 / SW;  // slots per warp
+    const int sw = s < S ? s : S;
+    for (int d = 1; d < sw; d *= 2) {
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, d * SW);
+        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, d * SW);
+    }
+    if (s > S) {
+        const int parts = s / S;
+        if (sub % S == 0) red[(row * parts + sub / S) * SW + lane] = acc;
+        __syncthreads();
+        if (sub == 0) {
+            acc = red[(row * parts) * SW + lane];
+            for (int w = 1; w < parts; ++w) {
+                const Vec2<T> v = red[(row * parts + w) * SW + lane];
+                acc.x += v.x;
+                acc.y += v.y;
+            }
+        }
+    }
+    return acc;
+}
+
+// ---------------------------------------------------------------------------------------
+// numeric block LU (left-looking Crout), level by level
 // ---------------------------------------------------------------------------------------
 template <typename T, int SW>
-__global__ void k_factor(PlanDev P, BatchDev B) {
-    const int g = blockIdx.x;
+__global__ void __launch_bounds__(1024) k_factor(PlanDev P, BatchDev B, int split_slots) {
+    const LevelCta cta;
+    const int g = cta.g;
     if (!B.gsolve[g] || (B.gfactor && !B.gfactor[g])) return;
+    __shared__ int fa_buf[LV_MAX + 1], fb_buf[LV_MAX + 1];
+    const int* fa = level_bounds(P.fa_ptr, P.n_levels, fa_buf);
+    const int* fb = level_bounds(P.fb_ptr, P.n_levels, fb_buf);
     Blk<T>* F = reinterpret_cast<Blk<T>*>(B.F) + (size_t)g * P.n_slots * SW;
     const int lane = threadIdx.x % SW;
-    const int e0 = threadIdx.x / SW, ne = blockDim.x / SW;
+    const int e0 = (cta.rank * blockDim.x + threadIdx.x) / SW, ne = cta.nc * blockDim.x / SW;
     bool bad = false;
-    if (B.lvl_ts) lvl_stamp(B, P.n_levels, 0, g, 0);
+    if (B.lvl_ts) lvl_stamp(B, P.n_levels, 0, g, 0, cta.rank);
+    __syncthreads();
     for (int h = 0; h < P.n_levels; ++h) {
-        const int ta = P.fa_ptr[h], tb = P.fa_ptr[h + 1];
+        const int ta = fa[h], tb = fa[h + 1];
+        const int s = split_slots ? min(split_factor(tb - ta, split_slots), 32 / SW) : 1;
+        if (s > 1) {
+            // narrow levels: s neighbouring threads share a target's pairs (the longest lists, 20
+            // to 40 pairs, set the level's latency)
+            const int sub = e0 % s, wl = e0 % (32 / SW);
+            for (int e = e0; e - wl < (tb - ta) * s; e += ne) {
+                const bool on = e < (tb - ta) * s;
+                const int4 tg = on ? P.targets[ta + e / s] : make_int4(0, 0, 0, 0);
+                Blk<T> acc = on && sub == 0 && (tg.w & 2) ? ldb(F + (size_t)tg.x * SW + lane) : Blk<T>{0, 0, 0, 0};
+#pragma unroll 4
+                for (int p = tg.y + sub; p < tg.z; p += s) {
+                    const int2 pr = P.pairs[p];
+                    msub(acc, ldb(F + (size_t)pr.x * SW + lane), ldb(F + (size_t)pr.y * SW + lane));
+                }
+                for (int d = SW; d < s * SW; d <<= 1) {
+                    acc.a += __shfl_xor_sync(0xffffffffu, acc.a, d);
+                    acc.b += __shfl_xor_sync(0xffffffffu, acc.b, d);
+                    acc.c += __shfl_xor_sync(0xffffffffu, acc.c, d);
+                    acc.d += __shfl_xor_sync(0xffffffffu, acc.d, d);
+                }
+                if (on && sub == 0) {
+                    if (tg.w & 1) {
+                        bool ok;
+                        acc = inv2(acc, ok);
+                        bad |= !ok;
+                    }
+                    stb(F + (size_t)tg.x * SW + lane, acc);
+                }
+            }
+        }
         // two targets per worker at a time (targets of one level are independent), so that
         // their gathers overlap in memory
-        for (int t = ta + e0; t < tb; t += 2 * ne) {
+        for (int t = s > 1 ? tb : ta + e0; t < tb; t += 2 * ne) {
             const bool two = t + ne < tb;
             const int4 tg = P.targets[t];
             const int4 tg2 = two ? P.targets[t + ne] : make_int4(0, 0, 0, 0);
@@ -589,19 +699,19 @@ __global__ void k_factor(PlanDev P, BatchDev B) {
                 stb(F + (size_t)tg2.x * SW + lane, acc2);
             }
         }
-        __syncthreads();
-        const int sa = P.fb_ptr[h], sb = P.fb_ptr[h + 1];
+        cta.sync();
+        const int sa = fb[h], sb = fb[h + 1];
         if (sb > sa) {
             for (int t = sa + e0; t < sb; t += ne) {
                 const int2 sc = P.scale[t];
                 Blk<T>* Lp = F + (size_t)sc.x * SW + lane;
                 stb(Lp, mul(ldb(Lp), ldb(F + (size_t)sc.y * SW + lane)));
             }
-            __syncthreads();
+            cta.sync();
         }
-        if (B.lvl_ts) lvl_stamp(B, P.n_levels, 0, g, h + 1);
+        if (B.lvl_ts) lvl_stamp(B, P.n_levels, 0, g, h + 1, cta.rank);
     }
-    if (B.lvl_ts) lvl_stamp(B, P.n_levels, 0, g, P.n_levels + 1);
+    if (B.lvl_ts) lvl_stamp(B, P.n_levels, 0, g, P.n_levels + 1, cta.rank);
     if (bad) B.singular[g * SW + lane] = 1;
 }
 
@@ -1284,63 +1394,44 @@ __host__ __forceinline__ size_t dense_solve_smem(int n_tail, size_t esz) {
 // node gathers its sparse contributions; U x = y over the sparse levels (descending) once
 // the dense tail is solved.  x is written as FP64 (optionally added to `out`).
 // ---------------------------------------------------------------------------------------
-// Levels with few nodes split every row over s sub-slots (s a power of two, up to 32): the
-// sub-slots of one warp reduce with shuffles, the warps of one row through shared memory.
-// split_factor: the largest s <= 32 with c * s <= ne (at least 1).
-__device__ __forceinline__ int split_factor(int c, int ne) {
-    int s = 1;
-    while (s < 32 && c * s * 2 <= ne) s *= 2;
-    return s;
-}
-
-// Sum `acc` over the s sub-slots of each row (slot e0 = row * s + sub); the result is valid in
-// sub-slot 0.  Every thread of the block calls this (uniform s).
-template <typename T, int SW>
-__device__ __forceinline__ Vec2<T> split_reduce(Vec2<T> acc, int s, int sub, int row, int lane,
-                                                Vec2<T>* red) {
-    constexpr int S = 32 / SW;  // slots per warp
-    const int sw = s < S ? s : S;
-    for (int d = 1; d < sw; d *= 2) {
-        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, d * SW);
-        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, d * SW);
-    }
-    if (s > S) {
-        const int parts = s / S;
-        if (sub % S == 0) red[(row * parts + sub / S) * SW + lane] = acc;
-        __syncthreads();
-        if (sub == 0) {
-            acc = red[(row * parts) * SW + lane];
-            for (int w = 1; w < parts; ++w) {
-                const Vec2<T> v = red[(row * parts + w) * SW + lane];
-                acc.x += v.x;
-                acc.y += v.y;
-            }
-        }
-    }
-    return acc;
-}
-
-template <typename T, int SW>
-__global__ void k_solve_fwd(PlanDev P, BatchDev B, const double2* __restrict__ rhs,
+// Forward: L y = b, or with TR (the adjoint) U^T y = b, over the sparse levels, then every tail
+// node gathers its sparse contributions.
+template <typename T, int SW, bool TR>
+__global__ void __launch_bounds__(1024) k_solve_fwd(PlanDev P, BatchDev B, const double2* __restrict__ rhs,
                             int refine_pass) {
-    const int g = blockIdx.x;
+    const LevelCta cta;
+    const int g = cta.g;
     if (!B.gsolve[g] || (refine_pass && B.grefine && !B.grefine[g])) return;
     __shared__ Vec2<T> red[256];  // (blockDim / (32 / SW)) partial sums, <= 256 for SW <= 8
+    __shared__ int lv_buf[LV_MAX + 1];
+    const int* lv = level_bounds(P.level_ptr, P.n_levels, lv_buf);
     const Blk<T>* F = reinterpret_cast<const Blk<T>*>(B.F) + (size_t)g * P.n_slots * SW;
+    const Blk<T>* E = F + (TR ? (size_t)P.nnz_l * SW : 0);  // U(k, j) sits nnz_l past L(j, k)
     Vec2<T>* X = reinterpret_cast<Vec2<T>*>(B.X) + (size_t)g * P.nb * SW;
     const double2* R = rhs + (size_t)g * P.nb * SW;
-    const int lane = threadIdx.x % SW;
-    const int e0 = threadIdx.x / SW, ne = blockDim.x / SW;
-    if (B.lvl_ts) lvl_stamp(B, P.n_levels, 1, g, 0);
+    const int lane = threadIdx.x % SW, n1 = blockDim.x / SW;  // slots of one CTA
+    const int e1 = threadIdx.x / SW;
+    const int e0 = cta.rank * n1 + e1, ne = cta.nc * n1;
+    auto entry = [&](Vec2<T>& acc, int2 r) {
+        const Blk<T> m = ldb(E + (size_t)r.x * SW + lane);
+        const Vec2<T> x = ldv(X + (size_t)r.y * SW + lane);
+        if (TR) msubtv(acc, m, x);
+        else msubv(acc, m, x);
+    };
+    auto finish = [&](int k, Vec2<T> acc) {
+        if (TR) acc = multv(ldb(F + (size_t)k * SW + lane), acc);
+        stv(X + (size_t)k * SW + lane, acc);
+    };
+    if (B.lvl_ts) lvl_stamp(B, P.n_levels, 1, g, 0, cta.rank);
+    __syncthreads();
     for (int h = 0; h < P.n_levels; ++h) {
-        const int lb = P.level_ptr[h], c = P.level_ptr[h + 1] - lb;
-        const int s = split_factor(c, ne);
+        const int lb = lv[h], c = lv[h + 1] - lb;
+        const int s = split_factor(c, n1);
         if (s == 1) {
             // two nodes per worker at a time (nodes of one level are independent)
-            for (int t = lb + e0; t < lb + c; t += 2 * ne) {
-                const bool two = t + ne < lb + c;
-                const int k = P.level_nodes[t];
-                const int k2 = two ? P.level_nodes[t + ne] : k;
+            for (int k = lb + e0; k < lb + c; k += 2 * ne) {
+                const bool two = k + ne < lb + c;
+                const int k2 = two ? k + ne : k;
                 const double2 b = R[(size_t)k * SW + lane];
                 const double2 b2 = R[(size_t)k2 * SW + lane];
                 Vec2<T> acc = {(T)b.x, (T)b.y}, acc2 = {(T)b2.x, (T)b2.y};
@@ -1349,43 +1440,35 @@ __global__ void k_solve_fwd(PlanDev P, BatchDev B, const double2* __restrict__ r
                 const int nb = min(qe - qa, qe2 - qa2);
 #pragma unroll 2
                 for (int i = 0; i < nb; ++i) {
-                    const int2 r = P.rlist[qa + i];
-                    const int2 r2 = P.rlist[qa2 + i];
-                    msubv(acc, ldb(F + (size_t)r.x * SW + lane), ldv(X + (size_t)r.y * SW + lane));
-                    msubv(acc2, ldb(F + (size_t)r2.x * SW + lane), ldv(X + (size_t)r2.y * SW + lane));
+                    const int2 r = P.rlist[qa + i], r2 = P.rlist[qa2 + i];
+                    entry(acc, r);
+                    entry(acc2, r2);
                 }
 #pragma unroll 4
-                for (int q = qa + nb; q < qe; ++q) {
-                    const int2 r = P.rlist[q];
-                    msubv(acc, ldb(F + (size_t)r.x * SW + lane), ldv(X + (size_t)r.y * SW + lane));
-                }
+                for (int q = qa + nb; q < qe; ++q) entry(acc, P.rlist[q]);
 #pragma unroll 4
-                for (int q = qa2 + nb; q < qe2; ++q) {
-                    const int2 r = P.rlist[q];
-                    msubv(acc2, ldb(F + (size_t)r.x * SW + lane), ldv(X + (size_t)r.y * SW + lane));
-                }
-                stv(X + (size_t)k * SW + lane, acc);
-                if (two) stv(X + (size_t)k2 * SW + lane, acc2);
+                for (int q = qa2 + nb; q < qe2; ++q) entry(acc2, P.rlist[q]);
+                finish(k, acc);
+                if (two) finish(k2, acc2);
             }
-        } else {
-            const int j = e0 / s, sub = e0 % s;
-            const int k = j < c ? P.level_nodes[lb + j] : 0;
+        } else if (cta.rank == 0) {
+            const int j = e1 / s, sub = e1 % s;
+            const int k = lb + min(j, c - 1);
             Vec2<T> acc = {T(0), T(0)};
             if (j < c) {
 #pragma unroll 4
-                for (int q = P.rptr[k] + sub; q < P.rptr[k + 1]; q += s) {
-                    const int2 r = P.rlist[q];
-                    msubv(acc, ldb(F + (size_t)r.x * SW + lane), ldv(X + (size_t)r.y * SW + lane));
-                }
+                for (int q = P.rptr[k] + sub; q < P.rptr[k + 1]; q += s) entry(acc, P.rlist[q]);
             }
             acc = split_reduce<T, SW>(acc, s, sub, j, lane, red);
             if (j < c && sub == 0) {
                 const double2 b = R[(size_t)k * SW + lane];
-                stv(X + (size_t)k * SW + lane, Vec2<T>{(T)b.x + acc.x, (T)b.y + acc.y});
+                finish(k, Vec2<T>{(T)b.x + acc.x, (T)b.y + acc.y});
             }
         }
-        __syncthreads();
-        if (B.lvl_ts) lvl_stamp(B, P.n_levels, 1, g, h + 1);
+        // a level split over sub-slots fits one CTA: between two of them the others run ahead
+        if (s > 1 && h + 1 < P.n_levels && split_factor(lv[h + 2] - lv[h + 1], n1) > 1) cta.sync_solo();
+        else cta.sync();
+        if (B.lvl_ts) lvl_stamp(B, P.n_levels, 1, g, h + 1, cta.rank);
     }
     {
         // tail rows gather long sparse rows: 4 sub-slots per row (a shuffle reduction within
@@ -1397,10 +1480,7 @@ __global__ void k_solve_fwd(PlanDev P, BatchDev B, const double2* __restrict__ r
             Vec2<T> acc = {T(0), T(0)};
             if (k < P.nb) {
 #pragma unroll 4
-                for (int q = P.rptr[k] + sub; q < P.rptr[k + 1]; q += TS) {
-                    const int2 r = P.rlist[q];
-                    msubv(acc, ldb(F + (size_t)r.x * SW + lane), ldv(X + (size_t)r.y * SW + lane));
-                }
+                for (int q = P.rptr[k] + sub; q < P.rptr[k + 1]; q += TS) entry(acc, P.rlist[q]);
             }
             acc = split_reduce<T, SW>(acc, TS, sub, 0, lane, red);
             if (k < P.nb && sub == 0) {
@@ -1411,23 +1491,35 @@ __global__ void k_solve_fwd(PlanDev P, BatchDev B, const double2* __restrict__ r
     }
     if (B.lvl_ts) {
         __syncthreads();
-        lvl_stamp(B, P.n_levels, 1, g, P.n_levels + 1);
+        lvl_stamp(B, P.n_levels, 1, g, P.n_levels + 1, cta.rank);
     }
 }
 
-template <typename T, int SW>
-__global__ void k_solve_bwd(PlanDev P, BatchDev B, double2* out, int accumulate) {
-    const int g = blockIdx.x;
+// Backward: U x = y, or with TR L^T x = y, over the sparse levels (descending) once the dense tail
+// is solved; x written as FP64 (optionally added to `out`).
+template <typename T, int SW, bool TR>
+__global__ void __launch_bounds__(1024) k_solve_bwd(PlanDev P, BatchDev B, double2* out, int accumulate) {
+    const LevelCta cta;
+    const int g = cta.g;
     if (!B.gsolve[g] || (accumulate && B.grefine && !B.grefine[g])) return;
     __shared__ Vec2<T> red[256];
+    __shared__ int lv_buf[LV_MAX + 1];
+    const int* lv = level_bounds(P.level_ptr, P.n_levels, lv_buf);
     const Blk<T>* F = reinterpret_cast<const Blk<T>*>(B.F) + (size_t)g * P.n_slots * SW;
+    const Blk<T>* E = F + ((size_t)P.nb + (TR ? 0 : P.nnz_l)) * SW;
     Vec2<T>* X = reinterpret_cast<Vec2<T>*>(B.X) + (size_t)g * P.nb * SW;
     double2* O = out + (size_t)g * P.nb * SW;
-    const int lane = threadIdx.x % SW;
-    const int e0 = threadIdx.x / SW, ne = blockDim.x / SW;
-    const int Ub = P.nb + P.nnz_l;
+    const int lane = threadIdx.x % SW, n1 = blockDim.x / SW;
+    const int e1 = threadIdx.x / SW;
+    const int e0 = cta.rank * n1 + e1, ne = cta.nc * n1;
+    auto entry = [&](Vec2<T>& acc, int p) {
+        const Blk<T> m = ldb(E + (size_t)p * SW + lane);
+        const Vec2<T> x = ldv(X + (size_t)P.lidx[p] * SW + lane);
+        if (TR) msubtv(acc, m, x);
+        else msubv(acc, m, x);
+    };
     auto finish = [&](int k, Vec2<T> acc) {
-        const Vec2<T> x = mulv(ldb(F + (size_t)k * SW + lane), acc);
+        const Vec2<T> x = TR ? acc : mulv(ldb(F + (size_t)k * SW + lane), acc);
         stv(X + (size_t)k * SW + lane, x);
         double2* o = O + (size_t)k * SW + lane;
         if (accumulate) {
@@ -1437,16 +1529,16 @@ __global__ void k_solve_bwd(PlanDev P, BatchDev B, double2* out, int accumulate)
             *o = make_double2((double)x.x, (double)x.y);
         }
     };
-    if (B.lvl_ts) lvl_stamp(B, P.n_levels, 2, g, 0);
+    if (B.lvl_ts) lvl_stamp(B, P.n_levels, 2, g, 0, cta.rank);
+    __syncthreads();
     for (int h = P.n_levels - 1; h >= 0; --h) {
-        const int lb = P.level_ptr[h], c = P.level_ptr[h + 1] - lb;
-        const int s = split_factor(c, ne);
+        const int lb = lv[h], c = lv[h + 1] - lb;
+        const int s = split_factor(c, n1);
         if (s == 1) {
             // two nodes per worker at a time (nodes of one level are independent)
-            for (int t = lb + e0; t < lb + c; t += 2 * ne) {
-                const bool two = t + ne < lb + c;
-                const int k = P.level_nodes[t];
-                const int k2 = two ? P.level_nodes[t + ne] : k;
+            for (int k = lb + e0; k < lb + c; k += 2 * ne) {
+                const bool two = k + ne < lb + c;
+                const int k2 = two ? k + ne : k;
                 Vec2<T> acc = ldv(X + (size_t)k * SW + lane);
                 Vec2<T> acc2 = ldv(X + (size_t)k2 * SW + lane);
                 const int pa = P.lptr[k], pe = P.lptr[k + 1];
@@ -1454,34 +1546,23 @@ __global__ void k_solve_bwd(PlanDev P, BatchDev B, double2* out, int accumulate)
                 const int nb = min(pe - pa, pe2 - pa2);
 #pragma unroll 2
                 for (int i = 0; i < nb; ++i) {
-                    msubv(acc, ldb(F + (size_t)(Ub + pa + i) * SW + lane),
-                          ldv(X + (size_t)P.lidx[pa + i] * SW + lane));
-                    msubv(acc2, ldb(F + (size_t)(Ub + pa2 + i) * SW + lane),
-                          ldv(X + (size_t)P.lidx[pa2 + i] * SW + lane));
+                    entry(acc, pa + i);
+                    entry(acc2, pa2 + i);
                 }
 #pragma unroll 4
-                for (int p = pa + nb; p < pe; ++p) {
-                    msubv(acc, ldb(F + (size_t)(Ub + p) * SW + lane),
-                          ldv(X + (size_t)P.lidx[p] * SW + lane));
-                }
+                for (int p = pa + nb; p < pe; ++p) entry(acc, p);
 #pragma unroll 4
-                for (int p = pa2 + nb; p < pe2; ++p) {
-                    msubv(acc2, ldb(F + (size_t)(Ub + p) * SW + lane),
-                          ldv(X + (size_t)P.lidx[p] * SW + lane));
-                }
+                for (int p = pa2 + nb; p < pe2; ++p) entry(acc2, p);
                 finish(k, acc);
                 if (two) finish(k2, acc2);
             }
-        } else {
-            const int j = e0 / s, sub = e0 % s;
-            const int k = j < c ? P.level_nodes[lb + j] : 0;
+        } else if (cta.rank == 0) {
+            const int j = e1 / s, sub = e1 % s;
+            const int k = lb + min(j, c - 1);
             Vec2<T> acc = {T(0), T(0)};
             if (j < c) {
 #pragma unroll 4
-                for (int p = P.lptr[k] + sub; p < P.lptr[k + 1]; p += s) {
-                    msubv(acc, ldb(F + (size_t)(Ub + p) * SW + lane),
-                          ldv(X + (size_t)P.lidx[p] * SW + lane));
-                }
+                for (int p = P.lptr[k] + sub; p < P.lptr[k + 1]; p += s) entry(acc, p);
             }
             acc = split_reduce<T, SW>(acc, s, sub, j, lane, red);
             if (j < c && sub == 0) {
@@ -1489,10 +1570,11 @@ __global__ void k_solve_bwd(PlanDev P, BatchDev B, double2* out, int accumulate)
                 finish(k, Vec2<T>{xk.x + acc.x, xk.y + acc.y});
             }
         }
-        __syncthreads();
-        if (B.lvl_ts) lvl_stamp(B, P.n_levels, 2, g, P.n_levels - h);
+        if (s > 1 && h > 0 && split_factor(lv[h] - lv[h - 1], n1) > 1) cta.sync_solo();
+        else cta.sync();
+        if (B.lvl_ts) lvl_stamp(B, P.n_levels, 2, g, P.n_levels - h, cta.rank);
     }
-    if (B.lvl_ts) lvl_stamp(B, P.n_levels, 2, g, P.n_levels + 1);
+    if (B.lvl_ts) lvl_stamp(B, P.n_levels, 2, g, P.n_levels + 1, cta.rank);
 }
 
 // refinement residual: res = rhs - J dx with the FP64 Jacobian blocks
@@ -1694,43 +1776,6 @@ __global__ void k_adj_rhs(PlanDev P, BatchDev B, const double* __restrict__ dvm,
 }
 
 template <typename T, int SW>
-__global__ void k_solve_fwd_t(PlanDev P, BatchDev B, const double2* __restrict__ rhs) {
-    const int g = blockIdx.x;
-    if (!B.gsolve[g]) return;
-    const Blk<T>* F = reinterpret_cast<const Blk<T>*>(B.F) + (size_t)g * P.n_slots * SW;
-    Vec2<T>* X = reinterpret_cast<Vec2<T>*>(B.X) + (size_t)g * P.nb * SW;
-    const double2* R = rhs + (size_t)g * P.nb * SW;
-    const int lane = threadIdx.x % SW;
-    const int e0 = threadIdx.x / SW, ne = blockDim.x / SW;
-    for (int h = 0; h < P.n_levels; ++h) {
-        for (int t = P.level_ptr[h] + e0; t < P.level_ptr[h + 1]; t += ne) {
-            const int j = P.level_nodes[t];
-            const double2 b = R[(size_t)j * SW + lane];
-            Vec2<T> acc = {(T)b.x, (T)b.y};
-#pragma unroll 4
-            for (int q = P.rptr[j]; q < P.rptr[j + 1]; ++q) {
-                const int2 r = P.rlist[q];  // (L slot of (j,k), k); U(k,j) sits nnz_l further
-                msubtv(acc, ldb(F + (size_t)(r.x + P.nnz_l) * SW + lane),
-                       ldv(X + (size_t)r.y * SW + lane));
-            }
-            stv(X + (size_t)j * SW + lane, multv(ldb(F + (size_t)j * SW + lane), acc));
-        }
-        __syncthreads();
-    }
-    for (int j = P.ns + e0; j < P.nb; j += ne) {
-        const double2 b = R[(size_t)j * SW + lane];
-        Vec2<T> acc = {(T)b.x, (T)b.y};
-#pragma unroll 4
-        for (int q = P.rptr[j]; q < P.rptr[j + 1]; ++q) {
-            const int2 r = P.rlist[q];
-            msubtv(acc, ldb(F + (size_t)(r.x + P.nnz_l) * SW + lane),
-                   ldv(X + (size_t)r.y * SW + lane));
-        }
-        stv(X + (size_t)j * SW + lane, acc);
-    }
-}
-
-template <typename T, int SW>
 __global__ void __launch_bounds__(256) k_dense_solve_t(PlanDev P, BatchDev B, double2* out,
                                                        int accumulate) {
     const int q = blockIdx.x;
@@ -1810,37 +1855,6 @@ __global__ void __launch_bounds__(256) k_dense_solve_t(PlanDev P, BatchDev B, do
         } else {
             *o = make_double2((double)y[2 * i], (double)y[2 * i + 1]);
         }
-    }
-}
-
-template <typename T, int SW>
-__global__ void k_solve_bwd_t(PlanDev P, BatchDev B, double2* out, int accumulate) {
-    const int g = blockIdx.x;
-    if (!B.gsolve[g]) return;
-    const Blk<T>* F = reinterpret_cast<const Blk<T>*>(B.F) + (size_t)g * P.n_slots * SW;
-    Vec2<T>* X = reinterpret_cast<Vec2<T>*>(B.X) + (size_t)g * P.nb * SW;
-    double2* O = out + (size_t)g * P.nb * SW;
-    const int lane = threadIdx.x % SW;
-    const int e0 = threadIdx.x / SW, ne = blockDim.x / SW;
-    for (int h = P.n_levels - 1; h >= 0; --h) {
-        for (int t = P.level_ptr[h] + e0; t < P.level_ptr[h + 1]; t += ne) {
-            const int k = P.level_nodes[t];
-            Vec2<T> acc = ldv(X + (size_t)k * SW + lane);
-#pragma unroll 4
-            for (int p = P.lptr[k]; p < P.lptr[k + 1]; ++p) {
-                msubtv(acc, ldb(F + (size_t)(P.nb + p) * SW + lane),
-                       ldv(X + (size_t)P.lidx[p] * SW + lane));
-            }
-            stv(X + (size_t)k * SW + lane, acc);
-            double2* o = O + (size_t)k * SW + lane;
-            if (accumulate) {
-                const double2 old = *o;
-                *o = make_double2(old.x + (double)acc.x, old.y + (double)acc.y);
-            } else {
-                *o = make_double2((double)acc.x, (double)acc.y);
-            }
-        }
-        __syncthreads();
     }
 }
 
