@@ -416,7 +416,8 @@ __global__ void __launch_bounds__(256, 3) k_dlu_update_tc(BatchDev B, int N, int
     for (int j = 0; j < 16; ++j)
         if (j < rows_left) cv[j] = cbase[j * ld];
     const bool ok = tc_wait(smem_u32(&mbar), 0u);
-    if (__syncthreads_or(!ok)) {
+    const bool ran_out = __syncthreads_or(!ok);
+    if (ran_out) {
         // every thread agrees; wait once more (bounded) for the MMAs before freeing the memory
         tc_wait(smem_u32(&mbar), 0u);
         if (tid == 0) {
@@ -445,6 +446,8 @@ __global__ void __launch_bounds__(256, 3) k_dlu_update_tc(BatchDev B, int N, int
     __syncthreads();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(TC_N));
+    // the next panel's diagonal block lies in tile (0, 0) (its operands are no longer needed)
+    if (blockIdx.x == 0 && !ran_out) dlu_next_diag<float>(B, q, A, ld, N, k0 + W, reinterpret_cast<float*>(oper));
 }
 
 // Dynamic shared memory of k_dense_lu_tc.

@@ -14,6 +14,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstddef>
+
 #include "blocks.cuh"
 
 namespace gapk {
@@ -1055,6 +1057,20 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_dense_lu(BatchD
     if (tid == 0 && bad) B.singular[q] = 1;
 }
 
+constexpr int DLU_W = 32, DLU_TILE = 64, DLU_ROWS = 128;
+
+// The next diagonal block (k1, k1) by warp 0, its trailing block just updated by this CTA.
+// `buf`: shared memory of dlu_diag_elems elements.
+constexpr int DLU_DIAG_ELEMS = 2 * DLU_W * (DLU_W + 4) + DLU_W;
+template <typename T>
+__device__ __forceinline__ void dlu_next_diag(BatchDev const& B, int q, T* A, int ld, int N, int k1, T* buf) {
+    if (threadIdx.x < 32) {
+        if (dense_diag_block<T, DLU_W>(A, ld, k1, min(DLU_W, N - k1), buf, DLU_W + 4,
+                                       buf + DLU_W * (DLU_W + 4), buf + 2 * DLU_W * (DLU_W + 4)))
+            B.singular[q] = 1;
+    }
+}
+
 }  // namespace gapk
 
 #include "dense_lu_tc.cuh"
@@ -1098,44 +1114,69 @@ void launch_dense_lu(int W, int grid, size_t smem, cudaStream_t st, BatchDev con
 }
 
 // Split dense LU (the batch path): the same right-looking factorisation as k_dense_lu, one
-// panel of W = 32 columns at a time, as two launches per panel so that the rank-W trailing
-// update of every scenario is spread over many small CTAs instead of one CTA per scenario:
-//   k_dlu_panel  one CTA per scenario: steps A and B (diagonal block in one warp, whole L21 rows
-//                and U12 columns per thread), written back to the tail in global memory;
-//   k_dlu_update one CTA per (scenario, 64 x 64 tile of the trailing matrix): the tile's L21
-//                rows (transposed) and U12 columns staged in shared memory, 8x8 register tiles
-//                per thread, C -= L21 U12 in place.
+// panel of W = 32 columns at a time, as two launches per panel so that the panel's solves and
+// the rank-W trailing update of every scenario are spread over many small CTAs:
+//   k_dlu_solves one CTA per (scenario, 128 rows of L21 or columns of U12): a thread per row or
+//                column, the factored diagonal block staged in shared memory;
+//   k_dlu_update one CTA per (scenario, 64 x 64 tile of the trailing matrix): C -= L21 U12 in
+//                place; the CTA of tile (0, 0) then factors the next panel's diagonal block (one
+//                warp, dense_diag_block), which its tile alone holds, so that no launch waits for
+//                that serial step by itself.
 // No dynamic shared memory, so the tail size is limited only by device memory.
-constexpr int DLU_W = 32, DLU_TILE = 64;
+// With the diagonal block and all its solves in one CTA per scenario, the panels of a tail of
+// order 506 took 396 us for one FP64 scenario and 612 us for 256; the solves now take 112 and 458
+// us, the diagonal blocks are part of the updates (165 us for one scenario, 173 without them).
+// Bound by the solves' and the diagonal block's dependent steps for few scenarios, by the
+// re-reading of the trailing matrix for many.
+// The first diagonal block.
+template <typename T>
+__global__ void __launch_bounds__(32) k_dlu_diag(BatchDev B, int N) {
+    const int q = blockIdx.x;
+    if (q >= B.n_scen || !B.solving[q] || (B.gfactor && !B.gfactor[q / B.sw])) return;
+    __shared__ __align__(16) T buf[DLU_DIAG_ELEMS];
+    const int ld = dense_ld(N);
+    dlu_next_diag<T>(B, q, reinterpret_cast<T*>(B.Dt) + (size_t)q * N * ld, ld, N, 0, buf);
+}
 
 template <typename T>
-__global__ void __launch_bounds__(128) k_dlu_panel(BatchDev B, int N, int k0) {
+__global__ void __launch_bounds__(DLU_ROWS) k_dlu_solves(BatchDev B, int N, int k0) {
     constexpr int W = DLU_W;
-    const int q = blockIdx.x;
+    const int q = blockIdx.y;
     if (q >= B.n_scen || !B.solving[q] || (B.gfactor && !B.gfactor[q / B.sw])) return;
     const int ld = dense_ld(N);
     T* A = reinterpret_cast<T*>(B.Dt) + (size_t)q * N * ld;
     __shared__ __align__(16) T U11[W * (W + 4)];  // transposed: U11[c][k], stride W + 4
     __shared__ __align__(16) T SL[W * (W + 4)];   // L11 row-major, stride W + 4
     __shared__ __align__(16) T SD[W];
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int w = min(W, N - k0);
-    const int n2 = N - k0 - w;
-    if (tid < 32) {
-        if (dense_diag_block<T, W>(A, ld, k0, w, U11, W + 4, SL, SD)) B.singular[q] = 1;
+    const int tid = threadIdx.x;
+    V4<T> blk[2];  // all of a thread's loads in flight together
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int e = tid + i * DLU_ROWS;
+        blk[i] = ld4(A + (size_t)(k0 + e / (W / 4)) * ld + k0 + (e % (W / 4)) * 4);
     }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int e = tid + i * DLU_ROWS, r = e / (W / 4), c = (e % (W / 4)) * 4;
+        st4(SL + r * (W + 4) + c, blk[i]);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            U11[(c + t) * (W + 4) + r] = blk[i].v[t];
+            if (r == c + t) SD[r] = T(1) / blk[i].v[t];
+        }
+    }
+    static_assert(W * W == 2 * 4 * DLU_ROWS);
     __syncthreads();
-    for (int it = tid; it < 2 * n2; it += nt) {
-        if (it < n2)
-            dense_l21_row<T, W>(A + (size_t)(k0 + W + it) * ld + k0, U11, W + 4, SD, nullptr);
-        else
-            dense_u12_col<T, W>(A + (size_t)k0 * ld + k0 + W + (it - n2), SL, ld);
-    }
+    const int n2 = N - k0 - W, it = blockIdx.x * DLU_ROWS + tid;
+    if (it < n2)
+        dense_l21_row<T, W>(A + (size_t)(k0 + W + it) * ld + k0, U11, W + 4, SD, nullptr);
+    else if (it < 2 * n2)
+        dense_u12_col<T, W>(A + (size_t)k0 * ld + k0 + W + (it - n2), SL, ld);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 4)
-    k_dlu_update(BatchDev B, int N, int k0, int tiles_j) {
+// FP32, CUDA cores: 64 threads, 8 x 8 values each.
+__global__ void __launch_bounds__(64, 8) k_dlu_update(BatchDev B, int N, int k0, int tiles_j) {
+    using T = float;
     constexpr int W = DLU_W, TS = DLU_TILE;
     const int q = blockIdx.y;
     if (q >= B.n_scen || !B.solving[q] || (B.gfactor && !B.gfactor[q / B.sw])) return;
@@ -1145,6 +1186,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 4)
     const int i0 = (blockIdx.x / tiles_j) * TS, j0 = (blockIdx.x % tiles_j) * TS;
     __shared__ __align__(16) T LT[W][TS];  // LT[c][r] = L21(i0 + r, c)
     __shared__ __align__(16) T UT[W][TS];  // UT[r][c] = U12(r, j0 + c)
+    __shared__ __align__(16) T diag[DLU_DIAG_ELEMS];
     const int tid = threadIdx.x;
     T* base = A + (size_t)(k0 + W) * ld + k0 + W;  // trailing matrix origin
     {
@@ -1173,44 +1215,122 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 4)
     }
     __syncthreads();
     const int r0 = (tid / 8) * 8, c0 = (tid % 8) * 8;
-    if (i0 + r0 >= n2 || j0 + c0 >= n2) return;
-    T acc[8][8];
+    if (i0 + r0 < n2 && j0 + c0 < n2) {
+        T acc[8][8];
 #pragma unroll
-    for (int ii = 0; ii < 8; ++ii) {
-        if (i0 + r0 + ii < n2) {
-            const T* row = base + (size_t)(i0 + r0 + ii) * ld + j0 + c0;
-            const V4<T> a = ld4(row), b = ld4(row + 4);
+        for (int ii = 0; ii < 8; ++ii) {
+            if (i0 + r0 + ii < n2) {
+                const T* row = base + (size_t)(i0 + r0 + ii) * ld + j0 + c0;
+                const V4<T> a = ld4(row), b = ld4(row + 4);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                acc[ii][c] = a.v[c];
-                acc[ii][c + 4] = b.v[c];
+                for (int c = 0; c < 4; ++c) {
+                    acc[ii][c] = a.v[c];
+                    acc[ii][c + 4] = b.v[c];
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) acc[ii][c] = T(0);
             }
-        } else {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) acc[ii][c] = T(0);
         }
-    }
 #pragma unroll 2
-    for (int r = 0; r < W; ++r) {
-        const V4<T> l0 = ld4(&LT[r][r0]), l1 = ld4(&LT[r][r0 + 4]);
-        const V4<T> u0 = ld4(&UT[r][c0]), u1 = ld4(&UT[r][c0 + 4]);
+        for (int r = 0; r < W; ++r) {
+            const V4<T> l0 = ld4(&LT[r][r0]), l1 = ld4(&LT[r][r0 + 4]);
+            const V4<T> u0 = ld4(&UT[r][c0]), u1 = ld4(&UT[r][c0 + 4]);
 #pragma unroll
-        for (int ii = 0; ii < 4; ++ii)
+            for (int ii = 0; ii < 4; ++ii)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                acc[ii][c] = fma(-l0.v[ii], u0.v[c], acc[ii][c]);
-                acc[ii][c + 4] = fma(-l0.v[ii], u1.v[c], acc[ii][c + 4]);
-                acc[ii + 4][c] = fma(-l1.v[ii], u0.v[c], acc[ii + 4][c]);
-                acc[ii + 4][c + 4] = fma(-l1.v[ii], u1.v[c], acc[ii + 4][c + 4]);
+                for (int c = 0; c < 4; ++c) {
+                    acc[ii][c] = fma(-l0.v[ii], u0.v[c], acc[ii][c]);
+                    acc[ii][c + 4] = fma(-l0.v[ii], u1.v[c], acc[ii][c + 4]);
+                    acc[ii + 4][c] = fma(-l1.v[ii], u0.v[c], acc[ii + 4][c]);
+                    acc[ii + 4][c + 4] = fma(-l1.v[ii], u1.v[c], acc[ii + 4][c + 4]);
+                }
+        }
+#pragma unroll
+        for (int ii = 0; ii < 8; ++ii) {
+            if (i0 + r0 + ii < n2) {
+                T* row = base + (size_t)(i0 + r0 + ii) * ld + j0 + c0;
+                st4(row, V4<T>{{acc[ii][0], acc[ii][1], acc[ii][2], acc[ii][3]}});
+                st4(row + 4, V4<T>{{acc[ii][4], acc[ii][5], acc[ii][6], acc[ii][7]}});
+            }
+        }
+    }
+    if (blockIdx.x == 0) {
+        __syncthreads();
+        dlu_next_diag<T>(B, q, A, ld, N, k0 + W, diag);
+    }
+}
+
+// FP64: 128 threads, 8 rows x 2 column pairs each; a warp's loads and stores of C cover 256
+// adjacent bytes of a row, L21 stays row-major in shared memory (a row's value is one broadcast
+// read).  256 tails of order 506: 2,858 -> 1,480 us (64 threads with 8 x 8 values each before, rows
+// of L21 staged a thread per row).
+__global__ void __launch_bounds__(128, 4) k_dlu_update64(BatchDev B, int N, int k0, int tiles_j) {
+    using T = double;
+    constexpr int W = DLU_W, TS = DLU_TILE;
+    const int q = blockIdx.y;
+    if (q >= B.n_scen || !B.solving[q] || (B.gfactor && !B.gfactor[q / B.sw])) return;
+    const int ld = dense_ld(N);
+    T* A = reinterpret_cast<T*>(B.Dt) + (size_t)q * N * ld;
+    const int n2 = N - k0 - W;
+    const int i0 = (blockIdx.x / tiles_j) * TS, j0 = (blockIdx.x % tiles_j) * TS;
+    struct Smem {
+        T Ls[TS][W + 2];  // L21(i0 + r, c)
+        T Us[W][TS];      // U12(r, j0 + c)
+    };
+    __shared__ __align__(16) Smem sm;
+    auto& Ls = sm.Ls;
+    auto& Us = sm.Us;
+    const int tid = threadIdx.x;
+    T* base = A + (size_t)(k0 + W) * ld + k0 + W;  // trailing matrix origin
+    // rows and columns past the matrix are left as they are: they feed values that are not stored
+    for (int e = tid; e < TS * (W / 2); e += 128) {
+        const int r = e / (W / 2), c = (e % (W / 2)) * 2;
+        if (i0 + r < n2) cp_async<16>(&Ls[r][c], A + (size_t)(k0 + W + i0 + r) * ld + k0 + c);
+    }
+    for (int e = tid; e < W * (TS / 2); e += 128) {
+        const int r = e / (TS / 2), c = (e % (TS / 2)) * 2;
+        // a pair that starts inside the matrix ends inside the padded row
+        if (j0 + c < n2) cp_async<16>(&Us[r][c], A + (size_t)(k0 + r) * ld + k0 + W + j0 + c);
+    }
+    // rows r0 .. r0 + 7, columns c0 + 32 j and the next, j = 0, 1
+    const int r0 = (tid / 16) * 8, c0 = (tid % 16) * 2;
+    double2 acc[8][2];
+#pragma unroll
+    for (int ii = 0; ii < 8; ++ii)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            acc[ii][j] = i0 + r0 + ii < n2 && j0 + c0 + 32 * j < n2
+                             ? *reinterpret_cast<const double2*>(base + (size_t)(i0 + r0 + ii) * ld + j0 + c0 + 32 * j)
+                             : make_double2(0.0, 0.0);
+    cp_async_wait_all();
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < W; ++k) {
+        double2 u[2];
+        double l[8];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) u[j] = *reinterpret_cast<const double2*>(&Us[k][c0 + 32 * j]);
+#pragma unroll
+        for (int ii = 0; ii < 8; ++ii) l[ii] = Ls[r0 + ii][k];
+#pragma unroll
+        for (int ii = 0; ii < 8; ++ii)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                acc[ii][j].x = fma(-l[ii], u[j].x, acc[ii][j].x);
+                acc[ii][j].y = fma(-l[ii], u[j].y, acc[ii][j].y);
             }
     }
 #pragma unroll
-    for (int ii = 0; ii < 8; ++ii) {
-        if (i0 + r0 + ii < n2) {
-            T* row = base + (size_t)(i0 + r0 + ii) * ld + j0 + c0;
-            st4(row, V4<T>{{acc[ii][0], acc[ii][1], acc[ii][2], acc[ii][3]}});
-            st4(row + 4, V4<T>{{acc[ii][4], acc[ii][5], acc[ii][6], acc[ii][7]}});
-        }
+    for (int ii = 0; ii < 8; ++ii)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            if (i0 + r0 + ii < n2 && j0 + c0 + 32 * j < n2)
+                *reinterpret_cast<double2*>(base + (size_t)(i0 + r0 + ii) * ld + j0 + c0 + 32 * j) = acc[ii][j];
+    if (blockIdx.x == 0) {
+        __syncthreads();
+        static_assert(offsetof(Smem, Us) == sizeof(Smem::Ls) && sizeof(Smem) >= DLU_DIAG_ELEMS * sizeof(T));
+        dlu_next_diag<T>(B, q, A, ld, N, k0 + W, &sm.Ls[0][0]);
     }
 }
 
@@ -1220,19 +1340,18 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 4)
 // blocks, mostly empty as tensor-core tiles, keep the 64 x 64 CUDA-core tiles.
 template <typename T>
 void launch_dense_lu_split(int grid, cudaStream_t st, BatchDev const& B, int N, bool tc) {
-    for (int k0 = 0; k0 < N; k0 += DLU_W) {
-        k_dlu_panel<T><<<grid, 128, 0, st>>>(B, N, k0);
+    k_dlu_diag<T><<<grid, 32, 0, st>>>(B, N);
+    for (int k0 = 0; k0 + DLU_W < N; k0 += DLU_W) {
         const int n2 = N - k0 - DLU_W;
-        if (n2 > 0) {
-            if constexpr (sizeof(T) == 4) {
-                if (tc && n2 >= TC_N) {
-                    const int tt = (n2 + TC_N - 1) / TC_N;
-                    k_dlu_update_tc<<<dim3(tt * tt, grid), 256, TC_OPER_BYTES, st>>>(B, N, k0, tt);
-                    continue;
-                }
-            }
-            const int tj = (n2 + DLU_TILE - 1) / DLU_TILE;
-            k_dlu_update<T><<<dim3(tj * tj, grid), DLU_TILE, 0, st>>>(B, N, k0, tj);
+        k_dlu_solves<T><<<dim3((2 * n2 + DLU_ROWS - 1) / DLU_ROWS, grid), DLU_ROWS, 0, st>>>(B, N, k0);
+        const int tj = (n2 + DLU_TILE - 1) / DLU_TILE;
+        if constexpr (sizeof(T) == 8) {
+            k_dlu_update64<<<dim3(tj * tj, grid), 128, 0, st>>>(B, N, k0, tj);
+        } else if (tc && n2 >= TC_N) {
+            const int tt = (n2 + TC_N - 1) / TC_N;
+            k_dlu_update_tc<<<dim3(tt * tt, grid), 256, TC_OPER_BYTES, st>>>(B, N, k0, tt);
+        } else {
+            k_dlu_update<<<dim3(tj * tj, grid), DLU_TILE, 0, st>>>(B, N, k0, tj);
         }
     }
 }
