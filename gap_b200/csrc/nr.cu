@@ -253,6 +253,7 @@ struct gapk_nr_batch_s {
     int dense_fused = 0;
     int level_ctas = 1;  // CTAs per lane group of the level-scheduled kernels
     int split_slots = 0; // k_factor's split_slots
+    int dense_ctas = 1;  // CTAs per scenario of the dense tail's solves
     DevBuf V, Sspec, Scalc, Y, F, A64, rhs, dx, res, X, Dt, mis, state, solving, singular,
         iters, status, fmis, gsolve, giter, grefine, gfactor, ctrl, tol;
     int dense_w = 0;          // panel width of the one-CTA-per-scenario dense LU (0: not used)
@@ -279,20 +280,37 @@ inline unsigned blocks_for(long items, int threads) {
     return static_cast<unsigned>((items + threads - 1) / threads);
 }
 
-// A level-scheduled kernel, b->level_ctas CTAs (one cluster) per lane group.
+// `units` clusters of nc CTAs (plain CTAs for nc = 1).
 template <typename K, typename... A>
-void launch_levels(gapk_nr_batch b, cudaStream_t st, K kernel, A... args) {
+void launch_clusters(int units, int nc, int threads, size_t smem, cudaStream_t st, K kernel, A... args) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute cluster{};
     cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim.x = b->level_ctas;
+    cluster.val.clusterDim.x = nc;
     cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(b->G * b->level_ctas);
-    cfg.blockDim = dim3(b->threads);
+    cfg.gridDim = dim3(units * nc);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = &cluster;
-    cfg.numAttrs = b->level_ctas > 1 ? 1 : 0;
+    cfg.numAttrs = nc > 1 ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+// A level-scheduled kernel, b->level_ctas CTAs per lane group.
+template <typename K, typename... A>
+void launch_levels(gapk_nr_batch b, cudaStream_t st, K kernel, A... args) {
+    launch_clusters(b->G, b->level_ctas, b->threads, 0, st, kernel, args...);
+}
+// The tail's two substitutions; k_dense_solve streams best when its CTAs fill the GPU.
+template <typename T, int SW, bool TR>
+void launch_dense_solve(gapk_nr_batch b, cudaStream_t st, double2* out, int acc) {
+    PlanDev const& P = b->plan->dev;
+    if (P.n_tail == 0) return;
+    const size_t smem = dense_solve_smem(P.n_tail, sizeof(T));
+    if (TR || b->dense_ctas > 1)
+        launch_clusters(b->G * SW, b->dense_ctas, DS_THREADS, smem, st, k_dense_solve_cl<T, SW, TR>, P, b->dev, out, acc);
+    else
+        k_dense_solve<T, SW><<<b->G * SW, 256, smem, st>>>(P, b->dev, out, acc);
 }
 
 template <typename T, int SW>
@@ -300,8 +318,7 @@ void launch_solve(gapk_nr_batch b, cudaStream_t st, const double2* rhs, double2*
     PlanDev const& P = b->plan->dev;
     BatchDev const& B = b->dev;
     launch_levels(b, st, k_solve_fwd<T, SW, false>, P, B, rhs, acc);
-    if (P.n_tail > 0)
-        k_dense_solve<T, SW><<<b->G * SW, 256, dense_solve_smem(P.n_tail, sizeof(T)), st>>>(P, B, out, acc);
+    launch_dense_solve<T, SW, false>(b, st, out, acc);
     launch_levels(b, st, k_solve_bwd<T, SW, false>, P, B, out, acc);
 }
 
@@ -459,8 +476,7 @@ struct KernelOp {
                 break;
             case 5: launch_levels(b, st, k_solve_fwd<T, SW, false>, P, B, (const double2*)B.rhs, 0); break;
             case 6:
-                if (P.n_tail > 0)
-                    k_dense_solve<T, SW><<<G * SW, 256, dense_solve_smem(P.n_tail, sizeof(T)), st>>>(P, B, B.dx, 0);
+                launch_dense_solve<T, SW, false>(b, st, B.dx, 0);
                 break;
             case 7: launch_levels(b, st, k_solve_bwd<T, SW, false>, P, B, B.dx, 0); break;
             case 8: k_update<SW><<<dim3(blocks_for((long)P.n_bus * SW, 256), G), 256, 0, st>>>(P, B); break;
@@ -475,8 +491,7 @@ void launch_solve_t(gapk_nr_batch b, cudaStream_t st, const double2* rhs, double
     PlanDev const& P = b->plan->dev;
     BatchDev const& B = b->dev;
     launch_levels(b, st, k_solve_fwd<T, SW, true>, P, B, rhs, 0);
-    if (P.n_tail > 0)
-        k_dense_solve_t<T, SW><<<b->G * SW, 256, 2 * P.n_tail * sizeof(T), st>>>(P, B, out, acc);
+    launch_dense_solve<T, SW, true>(b, st, out, acc);
     launch_levels(b, st, k_solve_bwd<T, SW, true>, P, B, out, acc);
 }
 
@@ -685,6 +700,19 @@ struct SmallOp {
         cudaLaunchKernelEx(&cfg, k_nr_small<T, CL>, b->plan->dev, b->dev, refine, r.together, passes);
     }
 };
+// Large tails need more shared memory for their vector than a launch gets without opting in (one
+// limit for every batch: the attribute is the kernel's, not the batch's).
+constexpr size_t DENSE_SOLVE_SMEM_MAX = 200 * 1024;
+template <typename T, int SW>
+struct DenseSolveAttributesOp {
+    static void run(cudaError_t* e) {
+        auto set = [](auto fn) {
+            return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DENSE_SOLVE_SMEM_MAX);
+        };
+        *e = set(k_dense_solve_cl<T, SW, false>);
+        if (*e == cudaSuccess) *e = set(k_dense_solve_cl<T, SW, true>);
+    }
+};
 template <typename T>
 cudaError_t small_attributes() {
     auto set = [](auto fn) {
@@ -865,6 +893,7 @@ int gapk_nr_batch_create(gapk_nr_plan p, int n_scen, const gapk_nr_batch_options
     const size_t G = (n_scen + lanes - 1) / lanes;
     b->G = static_cast<int>(G);
     b->level_ctas = level_ctas(b->G, b->dense_fused);
+    b->dense_ctas = level_ctas(b->G * lanes, b->dense_fused);
     b->split_slots = b->level_ctas >= 4 ? b->level_ctas * b->threads / lanes : 0;
     const size_t L = G * lanes;
     const size_t esz = b->precision == GAPK_PREC_FP64 ? 8 : 4;
@@ -889,11 +918,10 @@ int gapk_nr_batch_create(gapk_nr_plan p, int n_scen, const gapk_nr_batch_options
         // spread each scenario's trailing update over many CTAs and have no shared-memory
         // limit on the tail size.
         const size_t N = 2 * (size_t)h.n_tail;
-        const size_t smem_max = 232448 - 1024;  // opt-in shared memory per block, less static
         b->dense_w = 0;
         for (int w : {32, 16, 8}) {
             size_t bytes = dense_lu_elems((int)N, w) * esz;
-            if (bytes <= smem_max && (w < 32 || esz == 4 || N <= 200)) {
+            if (bytes <= DENSE_LU_SMEM_MAX && (w < 32 || esz == 4 || N <= 200)) {
                 b->dense_w = w;
                 b->dense_smem = bytes;
                 break;
@@ -912,10 +940,14 @@ int gapk_nr_batch_create(gapk_nr_plan p, int n_scen, const gapk_nr_batch_options
         cudaError_t e = cudaSuccess;
         if (!b->dense_split)
             e = b->precision == GAPK_PREC_FP64
-                    ? dense_lu_attributes<double>(b->dense_w, b->dense_smem, false)
-                    : dense_lu_attributes<float>(b->dense_w, b->dense_smem, b->dense_tc);
+                    ? dense_lu_attributes<double>(b->dense_w, false)
+                    : dense_lu_attributes<float>(b->dense_w, b->dense_tc);
         else if (b->dense_tc)
             e = split_lu_attributes();
+        // dynamic + k_dense_solve_cl's 19 KB of static shared memory past the 48 KB of any launch
+        const size_t vec = dense_solve_smem(h.n_tail, esz);
+        if (e == cudaSuccess && vec > 28 * 1024)
+            dispatch_tsw<DenseSolveAttributesOp>(b->precision, lanes, &e);
         if (e != cudaSuccess) {
             set_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
             return GAPK_ECUDA;
@@ -1641,7 +1673,7 @@ int noalloc_scratch_ptr(void** out) {
         void* p = nullptr;
         GAPK_CUDA_TRY(cudaGetSymbolAddress(&p, g_noalloc_scratch));
         for (int w : {32, 16, 8})
-            GAPK_CUDA_TRY(dense_lu_attributes<double>(w, 232448 - 1024, false));
+            GAPK_CUDA_TRY(dense_lu_attributes<double>(w, false));
         g_noalloc_ptr[dev] = p;
     }
     *out = g_noalloc_ptr[dev];
@@ -1703,7 +1735,7 @@ extern "C" int gapk_nr_solve_noalloc(gapk_nr_plan p, const gapk_nr_inputs* in,
         // the panel width rule of gapk_nr_batch_create for FP64 tails
         for (int w : {32, 16, 8}) {
             size_t bytes = dense_lu_elems((int)N, w) * 8;
-            if (bytes <= 232448 - 1024 && (w < 32 || N <= 200)) {
+            if (bytes <= DENSE_LU_SMEM_MAX && (w < 32 || N <= 200)) {
                 dense_w = w;
                 dense_smem = bytes;
                 break;

@@ -12,6 +12,7 @@
 //   Jacobian   :546-727  polar partial derivatives; |V| < 1e-6 replaced by 1 (:578)
 //   update     :438-504  damped (0.9) and clamped polar update (policy REFERENCE)
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstddef>
@@ -1079,9 +1080,11 @@ namespace gapk {
 
 // Host side: opt in to the kernel's shared memory and launch it for panel width W.  With `tc`
 // (FP32, W = 32) the tail is factorised by k_dense_lu_tc instead, the trailing update on the
-// tensor cores; its shared memory does not depend on N.
+// tensor cores; its shared memory does not depend on N.  k_dense_lu opts in to all that a block may
+// have: the attribute is the kernel's, and a batch with a smaller tail must not lower it.
+constexpr size_t DENSE_LU_SMEM_MAX = 232448 - 1024;  // opt-in shared memory per block, less static
 template <typename T>
-cudaError_t dense_lu_attributes(int W, size_t smem, bool tc) {
+cudaError_t dense_lu_attributes(int W, bool tc) {
     auto set = [&](auto fn, size_t bytes) {
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -1091,9 +1094,9 @@ cudaError_t dense_lu_attributes(int W, size_t smem, bool tc) {
         if (tc) return W == 32 ? set(k_dense_lu_tc, dense_lu_tc_smem()) : cudaErrorInvalidValue;
     }
     switch (W) {
-        case 32: return set(k_dense_lu<T, 32>, smem);
-        case 16: return set(k_dense_lu<T, 16>, smem);
-        case 8: return set(k_dense_lu<T, 8>, smem);
+        case 32: return set(k_dense_lu<T, 32>, DENSE_LU_SMEM_MAX);
+        case 16: return set(k_dense_lu<T, 16>, DENSE_LU_SMEM_MAX);
+        case 8: return set(k_dense_lu<T, 8>, DENSE_LU_SMEM_MAX);
     }
     return cudaErrorInvalidValue;
 }
@@ -1503,9 +1506,177 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 7 : 4) k_dense_solve(Pla
     }
 }
 
-// Dynamic shared memory of k_dense_solve / k_dense_solve_t: the tail vector, padded to ld.
+// Dynamic shared memory of the dense solves: the tail vector, padded to whole blocks of 32.
 __host__ __forceinline__ size_t dense_solve_smem(int n_tail, size_t esz) {
-    return (size_t)dense_ld(2 * n_tail) * esz;
+    return (size_t)((2 * n_tail + 31) / 32 * 32) * esz;
+}
+
+// The same two substitutions with a cluster of CTAs per scenario, for batches of few scenarios
+// (one CTA streams the factor at 10 to 100 GB/s: every block of 32 waits for its dot products),
+// and the transposed ones of the adjoint.  Right-looking by blocks of 32:
+// block b belongs to CTA b % nc, which solves its triangle (one warp, reciprocals of the diagonal
+// taken beforehand) and sends the 32 values to every CTA; after a cluster barrier each CTA takes
+// them out of the rows of its own blocks, whose factor entries it has already loaded.  Every
+// value's sum is formed block by block in four parts, whatever the cluster's size.
+// TR: U^T w = y and L^T x = w, a thread per column instead of four threads per row.
+// Bound by the chain of blocks, 2 to 2.4 us each (triangle, cluster barrier, update).  One FP64
+// tail of order 506: 158 -> 79 us with 8 CTAs; 8 FP32 tails of order 1,424: 659 -> 176 us; the
+// transposed solves of 256 FP64 tails, column by column before: 991 -> 242 us.
+constexpr int DS_THREADS = 256;
+
+template <typename T, int SW, bool TR>
+__global__ void __launch_bounds__(DS_THREADS) k_dense_solve_cl(PlanDev P, BatchDev B, double2* out,
+                                                               int accumulate) {
+    namespace cg = cooperative_groups;
+    const LevelCta cta;
+    const int q = cta.g, nc = cta.nc, rank = cta.rank;
+    if (q >= B.n_scen || !B.solving[q]) return;
+    const int g = q / SW, lane = q % SW;
+    if (accumulate && B.grefine && !B.grefine[g]) return;
+    const int N = 2 * P.n_tail, ld = dense_ld(N), nblk = (N + 31) / 32;
+    const T* A = reinterpret_cast<const T*>(B.Dt) + (size_t)q * N * ld;
+    Vec2<T>* X = reinterpret_cast<Vec2<T>*>(B.X) + (size_t)g * P.nb * SW;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    T* y = reinterpret_cast<T*>(smraw);  // [32 * nblk], kept up to date for this CTA's blocks
+    __shared__ T tri[2][32][33], rdiag[2][32], sol[2][32], red[4][64];
+    const int tid = threadIdx.x, wid = tid >> 5, ln = tid & 31;
+    for (int i = tid; i < 16 * nblk; i += DS_THREADS) {
+        const Vec2<T> v = i < P.n_tail ? ldv(X + (size_t)(P.ns + i) * SW + lane) : Vec2<T>{T(0), T(0)};
+        y[2 * i] = v.x;
+        y[2 * i + 1] = v.y;
+    }
+    // block b's triangle (transposed for TR; the identity past the matrix) and its diagonal, by
+    // the threads from t0 on (all loads before the first store)
+    auto stage = [&](int b, bool unit, T (*tri)[33], T* rdiag, int t0) {
+        T a[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            const int e = tid - t0 + k * (DS_THREADS - t0), i = 32 * b + (e >> 5), j = 32 * b + (e & 31);
+            a[k] = (e >> 5) == (e & 31) ? T(1) : T(0);
+            if (e < 32 * 32 && i < N && j < N) a[k] = A[(size_t)i * ld + j];
+        }
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            const int e = tid - t0 + k * (DS_THREADS - t0), r = e >> 5, c = e & 31;
+            if (e >= 32 * 32) break;
+            if (TR) tri[c][r] = a[k];
+            else tri[r][c] = a[k];
+            if (r == c) rdiag[r] = unit ? T(1) : T(1) / a[k];
+        }
+    };
+    static_assert(5 * (DS_THREADS - 32) >= 32 * 32);
+    for (int sweep = 0; sweep < 2; ++sweep) {  // the lower triangle ascending, the upper descending
+        const bool up = sweep == 1, unit = up == TR;
+        const int top = rank + (nblk - 1 - rank) / nc * nc;  // this CTA's last block
+        int buf = 0;  // this CTA's next triangle is in tri[buf]
+        if (rank < nblk) stage(up ? top : rank, unit, tri[0], rdiag[0], 0);
+        __syncthreads();
+        for (int step = 0; step < nblk; ++step) {
+            const int b = up ? nblk - 1 - step : step;
+            const bool own = b % nc == rank;
+            // this CTA's remaining blocks: first, first + nc, ..., count of them
+            const int first = up ? rank : b + 1 + ((rank - b - 1) % nc + nc) % nc;
+            const int count = up ? (b - rank + nc - 1) / nc : (nblk - first + nc - 1) / nc;
+            // the 8 entries of this thread's part of a row or column, NP of them ahead of the
+            // barrier: nothing here depends on the solution (masked only where they are used, so
+            // that no thread waits for them before)
+            constexpr int NP = 4;
+            T pre[NP][8];
+            auto fetch = [&](int item, T (&a)[8]) {
+                const int blk = first + nc * (item >> 5);
+#pragma unroll
+                for (int t = 0; t < 8; ++t) a[t] = T(0);
+                if ((item >> 5) >= count) return;
+                if (TR) {
+                    const int col = 32 * blk + (item & 31), r = 32 * b + 8 * (tid >> 6);
+#pragma unroll
+                    for (int t = 0; t < 8; ++t)
+                        if (r + t < N && col < N) a[t] = A[(size_t)(r + t) * ld + col];
+                } else {
+                    const int row = 32 * blk + (item & 31), c = 32 * b + 8 * (tid & 3);
+                    if (row < N && c < ld) {
+                        const V4<T> u = ld4(A + (size_t)row * ld + c), w = ld4(A + (size_t)row * ld + c + 4);
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) {
+                            a[t] = u.v[t];
+                            a[t + 4] = w.v[t];
+                        }
+                    }
+                }
+            };
+            const int item0 = TR ? tid & 63 : tid >> 2;
+#pragma unroll
+            for (int p = 0; p < NP; ++p) fetch(item0 + 64 * p, pre[p]);
+            if (own && wid == 0) {
+                T v = y[32 * b + ln], m[32];
+                const T rd = rdiag[buf][ln];
+                if (up) {
+#pragma unroll
+                    for (int j = 31; j >= 0; --j) m[j] = ln < j ? -tri[buf][ln][j] : T(0);
+#pragma unroll
+                    for (int j = 31; j >= 0; --j) {
+                        if (ln == j) v *= rd;
+                        v = fma(m[j], __shfl_sync(0xffffffffu, v, j), v);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) m[j] = ln > j ? -tri[buf][ln][j] : T(0);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        if (ln == j) v *= rd;
+                        v = fma(m[j], __shfl_sync(0xffffffffu, v, j), v);
+                    }
+                }
+                y[32 * b + ln] = v;
+                if (nc == 1) sol[step & 1][ln] = v;
+                else
+                    for (int r = 0; r < nc; ++r) *cg::this_cluster().map_shared_rank(&sol[step & 1][ln], r) = v;
+            }
+            if (own) {
+                // meanwhile the other warps fetch this CTA's next triangle
+                const int next = up ? b - nc : b + nc;
+                if (wid > 0 && next >= 0 && next < nblk) stage(next, unit, tri[buf ^ 1], rdiag[buf ^ 1], 32);
+                buf ^= 1;
+            }
+            cta.sync();
+            const T* s = sol[step & 1] + 8 * (TR ? tid >> 6 : tid & 3);
+            const int left = TR ? 8 : N - 32 * b - 8 * (tid & 3);  // columns of this part in the matrix
+            auto take = [&](int item, T const (&a)[8]) {
+                T acc = T(0);
+#pragma unroll
+                for (int t = 0; t < 8; ++t) acc = fma(t < left ? a[t] : T(0), s[t], acc);
+                const int i = 32 * (first + nc * (item >> 5)) + (item & 31);
+                if (TR) {
+                    red[tid >> 6][tid & 63] = acc;
+                    __syncthreads();
+                    if (tid < 64 && (item >> 5) < count)
+                        y[i] -= (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
+                    __syncthreads();
+                } else {
+                    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+                    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+                    if ((tid & 3) == 0 && (item >> 5) < count) y[i] -= acc;
+                }
+            };
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+                if (64 * p < 32 * count) take(item0 + 64 * p, pre[p]);
+            for (int base = 64 * NP; base < 32 * count; base += 64) {
+                fetch(item0 + base, pre[0]);
+                take(item0 + base, pre[0]);
+            }
+            __syncthreads();
+        }
+    }
+    double2* O = out + (size_t)g * P.nb * SW;
+    for (int i = tid; i < P.n_tail; i += DS_THREADS) {
+        if ((i >> 4) % nc != rank) continue;
+        const int k = P.ns + i;
+        stv(X + (size_t)k * SW + lane, Vec2<T>{y[2 * i], y[2 * i + 1]});
+        double2* o = O + (size_t)k * SW + lane;
+        const double2 old = accumulate ? *o : make_double2(0.0, 0.0);
+        *o = make_double2(old.x + (double)y[2 * i], old.y + (double)y[2 * i + 1]);
+    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1892,89 +2063,6 @@ __global__ void k_adj_rhs(PlanDev P, BatchDev B, const double* __restrict__ dvm,
     const double gt = dva[(size_t)src * P.n_bus + i];
     const double gv = P.bus_type[i] == BUS_PQ ? dvm[(size_t)src * P.n_bus + i] : 0.0;
     B.rhs[((size_t)g * P.nb + node) * SW + lane] = make_double2(gt, gv);
-}
-
-template <typename T, int SW>
-__global__ void __launch_bounds__(256) k_dense_solve_t(PlanDev P, BatchDev B, double2* out,
-                                                       int accumulate) {
-    const int q = blockIdx.x;
-    if (q >= B.n_scen || !B.solving[q]) return;
-    const int g = q / SW, lane = q % SW;
-    const int N = 2 * P.n_tail, ld = dense_ld(N);
-    const T* A = reinterpret_cast<const T*>(B.Dt) + (size_t)q * N * ld;
-    Vec2<T>* X = reinterpret_cast<Vec2<T>*>(B.X) + (size_t)g * P.nb * SW;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    T* y = reinterpret_cast<T*>(smraw);
-    const int tid = threadIdx.x, wid = tid >> 5, ln = tid & 31, nw = blockDim.x >> 5;
-    for (int i = tid; i < P.n_tail; i += blockDim.x) {
-        const Vec2<T> v = ldv(X + (size_t)(P.ns + i) * SW + lane);
-        y[2 * i] = v.x;
-        y[2 * i + 1] = v.y;
-    }
-    __syncthreads();
-    // U^T w = y (lower triangular with U's diagonal)
-    for (int r0 = 0; r0 < N; r0 += 32) {
-        for (int rr = wid; rr < 32; rr += nw) {
-            const int row = r0 + rr;
-            if (row >= N) continue;
-            T acc = T(0);
-            for (int c = ln; c < r0; c += 32) acc = fma(A[(size_t)c * ld + row], y[c], acc);
-#pragma unroll
-            for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-            if (ln == 0) y[row] -= acc;
-        }
-        __syncthreads();
-        if (wid == 0) {
-            const int row = r0 + ln;
-            T v = row < N ? y[row] : T(0);
-            for (int j = 0; j < 32; ++j) {
-                if (r0 + j >= N) break;
-                if (ln == j) v = v / A[(size_t)row * ld + row];
-                const T vj = __shfl_sync(0xffffffffu, v, j);
-                if (ln > j && row < N) v = fma(-A[(size_t)(r0 + j) * ld + row], vj, v);
-            }
-            if (row < N) y[row] = v;
-        }
-        __syncthreads();
-    }
-    // L^T lam = w (unit upper triangular)
-    const int last = ((N - 1) / 32) * 32;
-    for (int r0 = last; r0 >= 0; r0 -= 32) {
-        const int r1 = min(r0 + 32, N);
-        for (int rr = wid; rr < 32; rr += nw) {
-            const int row = r0 + rr;
-            if (row >= N) continue;
-            T acc = T(0);
-            for (int c = r1 + ln; c < N; c += 32) acc = fma(A[(size_t)c * ld + row], y[c], acc);
-#pragma unroll
-            for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-            if (ln == 0) y[row] -= acc;
-        }
-        __syncthreads();
-        if (wid == 0) {
-            const int row = r0 + ln;
-            T v = row < N ? y[row] : T(0);
-            for (int j = 31; j >= 0; --j) {
-                if (r0 + j >= N) continue;
-                const T vj = __shfl_sync(0xffffffffu, v, j);
-                if (ln < j && row < N) v = fma(-A[(size_t)(r0 + j) * ld + row], vj, v);
-            }
-            if (row < N) y[row] = v;
-        }
-        __syncthreads();
-    }
-    double2* O = out + (size_t)g * P.nb * SW;
-    for (int i = tid; i < P.n_tail; i += blockDim.x) {
-        const int k = P.ns + i;
-        stv(X + (size_t)k * SW + lane, Vec2<T>{y[2 * i], y[2 * i + 1]});
-        double2* o = O + (size_t)k * SW + lane;
-        if (accumulate) {
-            const double2 old = *o;
-            *o = make_double2(old.x + (double)y[2 * i], old.y + (double)y[2 * i + 1]);
-        } else {
-            *o = make_double2((double)y[2 * i], (double)y[2 * i + 1]);
-        }
-    }
 }
 
 // res = g - J^T lam with the FP64 Jacobian blocks, by block column

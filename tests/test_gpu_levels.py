@@ -103,3 +103,44 @@ def test_adjoint_solves(scen):
     want_q = np.where(qeq >= 0, lam[qeq], 0.0)
     for got, want in ((p.grad[k], want_p), (q.grad[k], want_q)):
         assert np.max(np.abs(got.cpu().numpy() - want)) <= 1e-6 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("n,scen", [(700, 1), (300, 9)])
+def test_more_levels_than_the_bounds_buffer(n, scen):
+    """A line of buses eliminated in natural order: n - 1 levels of one node each, past and below
+    the 256 level bounds kept in shared memory plus one; FP64 flat start against the oracle."""
+    import torch
+
+    from gap_b200 import _native as N
+    from gap_b200.engine import NRBatch, NRPlan, YbusPlan, branch_params, shunt_params
+    from gap_b200.network import PQ, SLACK, Network
+
+    bt = np.full(n, PQ, np.int32)
+    bt[-1] = SLACK
+    p = np.full(n, -1e3)
+    p[-1] = 0.0
+    net = Network.build(bus_id=np.arange(n), u_rated=np.full(n, 10e3), bus_type=bt, p=p, q=0.3 * p,
+                        from_id=np.arange(n - 1), to_id=np.arange(1, n), r1=np.full(n - 1, 0.02),
+                        x1=np.full(n - 1, 0.02))
+    yp = YbusPlan.from_network(net)
+    y = yp.assemble(torch.as_tensor(branch_params(net), device="cuda"),
+                    torch.as_tensor(shunt_params(net), device="cuda"), mode=N.YBUS_REFERENCE,
+                    scale=10e3 ** 2 / 1e6)[0]
+    plan = NRPlan(yp.row_ptr, yp.col_idx, net.bus_type, jacobian="exact", ordering="natural", dense_min=-1)
+    assert plan.info["n_levels"] == n - 1
+    s = np.repeat(net.specified_power(1e6)[None], scen, axis=0)
+    b = NRBatch(plan, scen, precision="fp64", use_graph=False)
+    sd = torch.as_tensor(s, device="cuda")
+    v0 = torch.ones(n, dtype=torch.complex128, device="cuda")
+    b.stage_load(y, sd, v_init=v0)
+    for stage in ("mismatch", "jacobian", "factor", "solve"):
+        b.stage(stage)
+    dx = b.correction().cpu().numpy()
+    import scipy.sparse.linalg as spla
+
+    rp, ci, va = restate.ybus_reference(net)
+    ypu = va * (10e3 ** 2 / 1e6)
+    one = np.ones(n, complex)
+    J = restate.jacobian(rp, ci, ypu, one, net.bus_type, mode="exact", drop=False).tocsc()
+    want = spla.spsolve(J, -restate.mismatch(net.bus_type, restate.power_injections(rp, ci, ypu, one), s[0]))
+    assert np.max(np.abs(dx[-1] - want)) <= 1e-8 * np.max(np.abs(want))  # condition ~ n^2 ~ 5e5
