@@ -544,9 +544,12 @@ __global__ void __launch_bounds__(256) k_jfill(PlanDev P, BatchDev B) {
 // split over threads does not depend on the cluster: the solves split by the CTA size, the
 // factorisation by split_slots, the slots that the batch has when it runs alone (0: no splits).
 // Both are bound by the latency of dependent gathers, level after level.  30,000 buses x 8
-// scenarios (one group, FP32): factor 1,480 -> 363 us, forward 351 -> 130, backward 369 -> 177;
-// 10,000 buses x 256 in FP64 (32 groups, 256 -> 1024 threads a CTA): 2,249 -> 541, 948 -> 209,
-// 954 -> 232 us, of which the CTA size alone 1,041, 335 and 348.
+// scenarios (one group, FP32): factor 1,480 -> 374 us, forward 351 -> 124, backward 369 -> 152;
+// 10,000 buses x 256 in FP64 (32 groups, 256 -> 1024 threads a CTA): 2,249 -> 541, 948 -> 191,
+// 954 -> 212 us, of which the CTA size alone 1,041, 335 and 348; x 1024 in FP32 (128 groups of one
+// CTA): 843 -> 822, 315 -> 297, 330 -> 314.  In the narrow levels warps without rows go straight to
+// the barrier, and a split row's entries are loaded ROW_BATCH at a time (left to the compiler:
+// backward 222 us at 30,000 buses, 152 so).
 // ---------------------------------------------------------------------------------------
 struct LevelCta {
     int nc, rank, g;
@@ -578,15 +581,16 @@ __device__ __forceinline__ const int* level_bounds(const int* ptr, int n_levels,
 
 // Levels with few nodes split every row over s sub-slots (s a power of two, up to 32): the
 // sub-slots of one warp reduce with shuffles, the warps of one row through shared memory.
-// split_factor: the largest s <= 32 with c * s <= ne (at least 1).
-__device__ __forceinline__ int split_factor(int c, int ne) {
-    int s = 1;
-    while (s < 32 && c * s * 2 <= ne) s *= 2;
-    return s;
+// split_log: the largest l <= 5 with c << l <= ne (at least 0; c >= 1), s = 1 << l.
+__device__ __forceinline__ int split_log(int c, int ne) {
+    int l = __clz(c) - __clz(ne);
+    if (l > 0 && c << l > ne) --l;
+    return max(0, min(l, 5));
 }
 
-// Sum `acc` over the s sub-slots of each row (slot e0 = row * s + sub); the result is valid in
-// sub-slot 0.  Every thread of the block calls this (uniform s).
+// Sum `acc` over the s = 1 << ls sub-slots of each row (slot e0 = row * s + sub); the result is
+// valid in sub-slot 0.  Every thread of the block calls this (uniform s) unless s <= 32 / SW, where
+// whole warps may stay away.
 template <typename T, int SW>
 __device__ __forceinline__ Vec2<T> split_reduce(Vec2<T> acc, int s, int sub, int row, int lane,
                                                 Vec2<T>* red) {
@@ -615,6 +619,34 @@ __device__ __forceinline__ Vec2<T> split_reduce(Vec2<T> acc, int s, int sub, int
 // ---------------------------------------------------------------------------------------
 // numeric block LU (left-looking Crout), level by level
 // ---------------------------------------------------------------------------------------
+// Entries of a split row or target that a thread loads together (as many as 64 registers hold).
+template <typename T>
+constexpr int ROW_BATCH = sizeof(T) == 4 ? 4 : 2;
+
+// acc -= sum of the block products of pairs p, p + step, ... < pe, U pairs' blocks loaded together:
+// left to the compiler the loop keeps one or two in flight.
+template <typename T, int SW, int U>
+__device__ __forceinline__ void pair_sum(Blk<T>& acc, const Blk<T>* F, const int2* pairs, int lane, int p,
+                                         int pe, int step) {
+    for (; p + (U - 1) * step < pe; p += U * step) {
+        int2 r[U];
+        Blk<T> a[U], b[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) r[u] = pairs[p + u * step];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            a[u] = ldb(F + (size_t)r[u].x * SW + lane);
+            b[u] = ldb(F + (size_t)r[u].y * SW + lane);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) msub(acc, a[u], b[u]);
+    }
+    for (; p < pe; p += step) {
+        const int2 r = pairs[p];
+        msub(acc, ldb(F + (size_t)r.x * SW + lane), ldb(F + (size_t)r.y * SW + lane));
+    }
+}
+
 template <typename T, int SW>
 __global__ void __launch_bounds__(1024) k_factor(PlanDev P, BatchDev B, int split_slots) {
     const LevelCta cta;
@@ -626,25 +658,22 @@ __global__ void __launch_bounds__(1024) k_factor(PlanDev P, BatchDev B, int spli
     Blk<T>* F = reinterpret_cast<Blk<T>*>(B.F) + (size_t)g * P.n_slots * SW;
     const int lane = threadIdx.x % SW;
     const int e0 = (cta.rank * blockDim.x + threadIdx.x) / SW, ne = cta.nc * blockDim.x / SW;
+    constexpr int SW_LOG = SW == 8 ? 3 : SW == 4 ? 2 : SW == 2 ? 1 : 0;
     bool bad = false;
     if (B.lvl_ts) lvl_stamp(B, P.n_levels, 0, g, 0, cta.rank);
     __syncthreads();
     for (int h = 0; h < P.n_levels; ++h) {
         const int ta = fa[h], tb = fa[h + 1];
-        const int s = split_slots ? min(split_factor(tb - ta, split_slots), 32 / SW) : 1;
+        const int ls = split_slots && tb > ta ? min(split_log(tb - ta, split_slots), 5 - SW_LOG) : 0, s = 1 << ls;
         if (s > 1) {
             // narrow levels: s neighbouring threads share a target's pairs (the longest lists, 20
             // to 40 pairs, set the level's latency)
-            const int sub = e0 % s, wl = e0 % (32 / SW);
-            for (int e = e0; e - wl < (tb - ta) * s; e += ne) {
-                const bool on = e < (tb - ta) * s;
-                const int4 tg = on ? P.targets[ta + e / s] : make_int4(0, 0, 0, 0);
+            const int sub = e0 & (s - 1), wl = e0 % (32 / SW);
+            for (int e = e0; e - wl < (tb - ta) << ls; e += ne) {
+                const bool on = e < (tb - ta) << ls;
+                const int4 tg = on ? P.targets[ta + (e >> ls)] : make_int4(0, 0, 0, 0);
                 Blk<T> acc = on && sub == 0 && (tg.w & 2) ? ldb(F + (size_t)tg.x * SW + lane) : Blk<T>{0, 0, 0, 0};
-#pragma unroll 4
-                for (int p = tg.y + sub; p < tg.z; p += s) {
-                    const int2 pr = P.pairs[p];
-                    msub(acc, ldb(F + (size_t)pr.x * SW + lane), ldb(F + (size_t)pr.y * SW + lane));
-                }
+                pair_sum<T, SW, ROW_BATCH<T>>(acc, F, P.pairs, lane, tg.y + sub, tg.z, s);
                 for (int d = SW; d < s * SW; d <<= 1) {
                     acc.a += __shfl_xor_sync(0xffffffffu, acc.a, d);
                     acc.b += __shfl_xor_sync(0xffffffffu, acc.b, d);
@@ -746,8 +775,11 @@ __device__ __forceinline__ void st4(double* p, V4<double> const& a) {
     reinterpret_cast<double2*>(p)[1] = make_double2(a.v[2], a.v[3]);
 }
 
+// Two pairs' blocks in flight per thread, and the CTAs per SM that this leaves registers for: one
+// pair more costs resident warps.  10,000 buses: 1024 scenarios in FP32 1,250 -> 1,140 us (1 / 3 / 4
+// pairs: 1,335 / 1,398 / 1,464), 256 in FP64 608 -> 591 us (8 CTAs: 837).
 template <typename T, int SW>
-__global__ void __launch_bounds__(256) k_schur(PlanDev P, BatchDev B) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 6) k_schur(PlanDev P, BatchDev B) {
     const int g = blockIdx.y;
     if (!B.gsolve[g] || (B.gfactor && !B.gfactor[g])) return;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -757,11 +789,7 @@ __global__ void __launch_bounds__(256) k_schur(PlanDev P, BatchDev B) {
     const Blk<T>* F = reinterpret_cast<const Blk<T>*>(B.F) + (size_t)g * P.n_slots * SW;
     const int4 tg = P.schur[t];
     Blk<T> acc = (tg.w >> 30) ? ldb(F + (size_t)tg.x * SW + lane) : Blk<T>{0, 0, 0, 0};
-#pragma unroll 4
-    for (int p = tg.y; p < tg.z; ++p) {
-        const int2 pr = P.pairs[p];
-        msub(acc, ldb(F + (size_t)pr.x * SW + lane), ldb(F + (size_t)pr.y * SW + lane));
-    }
+    pair_sum<T, SW, 2>(acc, F, P.pairs, lane, tg.y, tg.z, 1);
     const int N = 2 * P.n_tail, ld = dense_ld(N);
     const int pos = tg.w & ((1 << 30) - 1);
     const int r = 2 * (pos / P.n_tail), c = 2 * (pos % P.n_tail);
@@ -1716,7 +1744,7 @@ __global__ void __launch_bounds__(1024) k_solve_fwd(PlanDev P, BatchDev B, const
     __syncthreads();
     for (int h = 0; h < P.n_levels; ++h) {
         const int lb = lv[h], c = lv[h + 1] - lb;
-        const int s = split_factor(c, n1);
+        const int ls = split_log(c, n1), s = 1 << ls;
         if (s == 1) {
             // two nodes per worker at a time (nodes of one level are independent)
             for (int k = lb + e0; k < lb + c; k += 2 * ne) {
@@ -1741,13 +1769,33 @@ __global__ void __launch_bounds__(1024) k_solve_fwd(PlanDev P, BatchDev B, const
                 finish(k, acc);
                 if (two) finish(k2, acc2);
             }
+        } else if (cta.rank == 0 && (threadIdx.x & ~31) / SW >= c << ls) {
+            if (s > 32 / SW) __syncthreads();  // a warp without rows: split_reduce's barrier
         } else if (cta.rank == 0) {
-            const int j = e1 / s, sub = e1 % s;
+            const int j = e1 >> ls, sub = e1 & (s - 1);
             const int k = lb + min(j, c - 1);
             Vec2<T> acc = {T(0), T(0)};
             if (j < c) {
-#pragma unroll 4
-                for (int q = P.rptr[k] + sub; q < P.rptr[k + 1]; q += s) entry(acc, P.rlist[q]);
+                int q = P.rptr[k] + sub;
+                const int qe = P.rptr[k + 1];
+                for (; q + (ROW_BATCH<T> - 1) * s < qe; q += ROW_BATCH<T> * s) {
+                    int2 r[ROW_BATCH<T>];
+                    Blk<T> m[ROW_BATCH<T>];
+                    Vec2<T> x[ROW_BATCH<T>];
+#pragma unroll
+                    for (int u = 0; u < ROW_BATCH<T>; ++u) r[u] = P.rlist[q + u * s];
+#pragma unroll
+                    for (int u = 0; u < ROW_BATCH<T>; ++u) {
+                        m[u] = ldb(E + (size_t)r[u].x * SW + lane);
+                        x[u] = ldv(X + (size_t)r[u].y * SW + lane);
+                    }
+#pragma unroll
+                    for (int u = 0; u < ROW_BATCH<T>; ++u) {
+                        if (TR) msubtv(acc, m[u], x[u]);
+                        else msubv(acc, m[u], x[u]);
+                    }
+                }
+                for (; q < qe; q += s) entry(acc, P.rlist[q]);
             }
             acc = split_reduce<T, SW>(acc, s, sub, j, lane, red);
             if (j < c && sub == 0) {
@@ -1756,7 +1804,7 @@ __global__ void __launch_bounds__(1024) k_solve_fwd(PlanDev P, BatchDev B, const
             }
         }
         // a level split over sub-slots fits one CTA: between two of them the others run ahead
-        if (s > 1 && h + 1 < P.n_levels && split_factor(lv[h + 2] - lv[h + 1], n1) > 1) cta.sync_solo();
+        if (s > 1 && h + 1 < P.n_levels && split_log(lv[h + 2] - lv[h + 1], n1) > 0) cta.sync_solo();
         else cta.sync();
         if (B.lvl_ts) lvl_stamp(B, P.n_levels, 1, g, h + 1, cta.rank);
     }
@@ -1823,7 +1871,7 @@ __global__ void __launch_bounds__(1024) k_solve_bwd(PlanDev P, BatchDev B, doubl
     __syncthreads();
     for (int h = P.n_levels - 1; h >= 0; --h) {
         const int lb = lv[h], c = lv[h + 1] - lb;
-        const int s = split_factor(c, n1);
+        const int ls = split_log(c, n1), s = 1 << ls;
         if (s == 1) {
             // two nodes per worker at a time (nodes of one level are independent)
             for (int k = lb + e0; k < lb + c; k += 2 * ne) {
@@ -1846,13 +1894,33 @@ __global__ void __launch_bounds__(1024) k_solve_bwd(PlanDev P, BatchDev B, doubl
                 finish(k, acc);
                 if (two) finish(k2, acc2);
             }
+        } else if (cta.rank == 0 && (threadIdx.x & ~31) / SW >= c << ls) {
+            if (s > 32 / SW) __syncthreads();  // a warp without rows: split_reduce's barrier
         } else if (cta.rank == 0) {
-            const int j = e1 / s, sub = e1 % s;
+            const int j = e1 >> ls, sub = e1 & (s - 1);
             const int k = lb + min(j, c - 1);
             Vec2<T> acc = {T(0), T(0)};
             if (j < c) {
-#pragma unroll 4
-                for (int p = P.lptr[k] + sub; p < P.lptr[k + 1]; p += s) entry(acc, p);
+                int p = P.lptr[k] + sub;
+                const int pe = P.lptr[k + 1];
+                for (; p + (ROW_BATCH<T> - 1) * s < pe; p += ROW_BATCH<T> * s) {
+                    int i[ROW_BATCH<T>];
+                    Blk<T> m[ROW_BATCH<T>];
+                    Vec2<T> x[ROW_BATCH<T>];
+#pragma unroll
+                    for (int u = 0; u < ROW_BATCH<T>; ++u) i[u] = P.lidx[p + u * s];
+#pragma unroll
+                    for (int u = 0; u < ROW_BATCH<T>; ++u) {
+                        m[u] = ldb(E + (size_t)(p + u * s) * SW + lane);
+                        x[u] = ldv(X + (size_t)i[u] * SW + lane);
+                    }
+#pragma unroll
+                    for (int u = 0; u < ROW_BATCH<T>; ++u) {
+                        if (TR) msubtv(acc, m[u], x[u]);
+                        else msubv(acc, m[u], x[u]);
+                    }
+                }
+                for (; p < pe; p += s) entry(acc, p);
             }
             acc = split_reduce<T, SW>(acc, s, sub, j, lane, red);
             if (j < c && sub == 0) {
@@ -1860,7 +1928,7 @@ __global__ void __launch_bounds__(1024) k_solve_bwd(PlanDev P, BatchDev B, doubl
                 finish(k, Vec2<T>{xk.x + acc.x, xk.y + acc.y});
             }
         }
-        if (s > 1 && h > 0 && split_factor(lv[h] - lv[h - 1], n1) > 1) cta.sync_solo();
+        if (s > 1 && h > 0 && split_log(lv[h] - lv[h - 1], n1) > 0) cta.sync_solo();
         else cta.sync();
         if (B.lvl_ts) lvl_stamp(B, P.n_levels, 2, g, P.n_levels - h, cta.rank);
     }
