@@ -646,10 +646,11 @@ int validate_inputs(gapk_nr_batch b, const gapk_nr_inputs* in) {
 // separate kernels are used), CTA size, whether a group's lanes decide together, and the shared
 // memory share of the SM.  Shapes are ranked by waves of CTAs, then by fewer lanes per CTA (a
 // lane more in a CTA lengthens every step of the level schedule), then by 256 threads over 128.
-// Against the separate kernels on transmission grids of 120 to 1,200 buses it takes 1/1.6 to 1/2.7
-// of their time while one wave holds the scenarios, 1/1.1 to 1/2.2 with two; with three waves it
-// still wins with FP32 factors (1/1.1 to 1/1.25) and where a CTA has an SM to itself (1/1.1), and
-// loses otherwise (300 buses x 1024 scenarios in FP64: 1051 us against 907).
+// Against the separate kernels on transmission grids of 120 to 1,200 buses it takes 1/1.6 to 1/3
+// of their time while one wave holds the scenarios and 1/1.1 to 1/1.6 with two.  With three it
+// still wins where an SM holds several FP32 CTAs (500 buses x 1024: 1,564 us against 1,610) or one
+// FP64 CTA (900 x 300: 1,507 / 1,583), and loses with several FP64 ones (300 x 1024: 982 / 856) or
+// one FP32 CTA, whose groups wait for each other across SMs (900 x 300: 1,481 / 1,365).
 SmallRun small_choice(gapk_nr_batch b, const gapk_nr_inputs* in) {
     auto const& h = b->plan->h;
     SmallRun r;
@@ -666,7 +667,7 @@ SmallRun small_choice(gapk_nr_batch b, const gapk_nr_inputs* in) {
             const long ctas = ((long)b->n_scen + cl - 1) / cl;
             const long waves = (ctas + 148 * per_sm - 1) / (148 * per_sm);
             const long cost = waves * (4 + cl);
-            if (waves > (esz == 4 || per_sm == 1 ? 3 : 2) || (r.cl && cost >= best_cost)) continue;
+            if (waves > ((esz == 4) == (per_sm > 1) ? 3 : 2) || (r.cl && cost >= best_cost)) continue;
             r.cl = cl;
             r.threads = thr;
             r.carveout = (int)std::min<long>(

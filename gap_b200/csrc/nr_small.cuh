@@ -13,9 +13,9 @@
 // rows padded with a zero block), so that a thread's next index is one load at a known address,
 // taken (from L1) before this level's barrier; the right-hand side is already in the solve
 // vector; and long rows are split over 2 or 4 threads (by the plan alone, so that results do not
-// depend on the launch shape).  A step still takes 0.45 us: about 150 dependent instructions.
-// 200-bus feeder, FP64, 10 iterations: 1,340 -> 590 us for one scenario, 1,590 -> 780 us for
-// 1024; a 500-bus grid, one scenario: 754 -> 380 us.
+// depend on the launch shape).  A step still takes 0.4 us, mostly dependent instructions.
+// 200-bus feeder, FP64, 10 iterations: 1,340 -> 450 us for one scenario, 1,590 -> 745 us for
+// 1024; a 500-bus grid, one scenario: 754 -> 358 us.
 //
 // Lanes per CTA: lanes are independent unless per-group refinement or reuse thresholds make a
 // group's lanes decide together; then the group's CTAs form a cluster and exchange their flags.
@@ -142,10 +142,18 @@ struct SmallCta {
         }
     }
 
-    // sum over the 1 << ls sub-slots of a row (neighbouring slots of one warp)
-    __device__ __forceinline__ T row_sum(T v, int ls) const {
-        for (int d = CL; d < (CL << ls); d <<= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-        return v;
+    // sum over the 1 << ls (1, 2 or 4) sub-slots of a row, neighbouring slots of one warp; the
+    // values' shuffles overlap
+    template <int NV>
+    __device__ __forceinline__ void row_sum(T (&v)[NV], int ls) const {
+        if (ls > 0) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], CL);
+        }
+        if (ls > 1) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 2 * CL);
+        }
     }
 
     // block LU level by level, then the tail's Schur complement and its dense LU; false when a
@@ -189,7 +197,9 @@ struct SmallCta {
                         acc = {acc.a + odd.a, acc.b + odd.b, acc.c + odd.c, acc.d + odd.d};
                     }
                 }
-                if (ls) acc = {row_sum(acc.a, ls), row_sum(acc.b, ls), row_sum(acc.c, ls), row_sum(acc.d, ls)};
+                T v[4] = {acc.a, acc.b, acc.c, acc.d};
+                row_sum(v, ls);
+                acc = {v[0], v[1], v[2], v[3]};
                 if (own) {
                     if (t & SMALL_DIAG) {
                         bool ok;
@@ -258,13 +268,21 @@ struct SmallCta {
         return ok;
     }
 
-    // One sweep over a level's rows: row k's entries (factor slot, node) summed, then done(k,
-    // sum).  `w`: this thread's first entry word, fetched a level ahead.
-    template <typename F>
-    __device__ __forceinline__ void level_rows(int lb, int rows, int base, int ml, uint2 w, F done) const {
+    // One sweep over a level's rows: x(k) takes the sum of row k's entries (factor slot, node) and,
+    // in the backward sweep, its pivot block.  `w`: this thread's first entry, fetched a level
+    // ahead; the row's own values are read before its entries, off the chain of the sums.
+    template <bool BWD>
+    __device__ __forceinline__ void level_rows(int lb, int rows, int base, int ml, uint2 w, bool accumulate) const {
         const int ls = ml >> 16, M = ml & 0xffff, W = rows << ls, wl = e0 & (32 / CL - 1);
         for (int e = e0; e - wl < W; e += ne) {
-            const bool on = e < W;
+            const bool on = e < W, own = on && (e & ((1 << ls) - 1)) == 0;
+            const int k = lb + (e >> ls);
+            Vec2<T> b = {T(0), T(0)};
+            Blk<T> pivot = {T(0), T(0), T(0), T(0)};
+            if (own) {
+                b = ldv(x(k));
+                if (BWD) pivot = ldb(f(k));
+            }
             Vec2<T> acc = {T(0), T(0)};
             if (on) {
                 const uint2* next = P.ell + base + e;
@@ -278,8 +296,14 @@ struct SmallCta {
                     acc = {acc.x + odd.x, acc.y + odd.y};
                 }
             }
-            if (ls) acc = {row_sum(acc.x, ls), row_sum(acc.y, ls)};
-            if (on && (e & ((1 << ls) - 1)) == 0) done(lb + (e >> ls), acc);
+            T v[2] = {acc.x, acc.y};
+            row_sum(v, ls);
+            if (own) {
+                Vec2<T> r = {b.x + v[0], b.y + v[1]};
+                if (BWD) r = mulv(pivot, r);
+                stv(x(k), r);
+                if (BWD) out(k, r, accumulate);
+            }
         }
         __syncthreads();
     }
@@ -295,10 +319,7 @@ struct SmallCta {
             const int4 ra = rec(h, 0), rc = rec(h, 2);
             const uint2 w = w1;
             if (h + 1 < n_fwd) first(rec(h + 1, 0).y, rec(h + 1, 2).x, rec(h + 1, 2).y);
-            level_rows(ra.x, ra.y, rc.x, rc.y, w, [&](int k, Vec2<T> a) {
-                const Vec2<T> b = ldv(x(k));
-                stv(x(k), Vec2<T>{b.x + a.x, b.y + a.y});
-            });
+            level_rows<false>(ra.x, ra.y, rc.x, rc.y, w, false);
         }
         if (P.n_tail > 0) {
             dense_solve(2 * P.n_tail);
@@ -311,12 +332,7 @@ struct SmallCta {
             const int4 ra = rec(h, 0), rc = rec(h, 2);
             const uint2 w = w1;
             if (h > 0) first(rec(h - 1, 0).y, rec(h - 1, 2).z, rec(h - 1, 2).w);
-            level_rows(ra.x, ra.y, rc.z, rc.w, w, [&](int k, Vec2<T> a) {
-                const Vec2<T> b = ldv(x(k));
-                const Vec2<T> r = mulv(ldb(f(k)), Vec2<T>{b.x + a.x, b.y + a.y});
-                stv(x(k), r);
-                out(k, r, accumulate);
-            });
+            level_rows<true>(ra.x, ra.y, rc.z, rc.w, w, accumulate);
         }
     }
     __device__ __forceinline__ void out(int k, Vec2<T> r, bool accumulate) const {
