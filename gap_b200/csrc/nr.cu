@@ -553,14 +553,19 @@ int default_threads(int nb, int lanes) {
     while (thr < 1024 && 8L * thr < (long)nb * lanes) thr *= 2;
     return thr;
 }
-// CTAs per lane group of the level-scheduled kernels: as many (a power of two, at most 8) as the
-// 148 SMs hold side by side with all `groups` running.  A batch that shares the GPU with
-// concurrent ones (dense_fused) takes two at most: four parts of 16 groups each took 26.5, 26.0,
-// 28.6 and 37.2 ms with 1, 2, 4 and 8.
-int level_ctas(int groups, int dense_fused) {
-    int nc = 1;
-    while (2 * nc <= (dense_fused ? 2 : 8) && groups * 2 * nc <= 148) nc *= 2;
-    return nc;
+// CTAs per lane group of the level-scheduled kernels, one cluster: 8 or 4 where that makes at most
+// 128 CTAs (16 clusters of 8 sit on the GPCs side by side; 18 groups of a 2,000-bus grid took 2.2 ms
+// with one CTA each, 2.7 ms with clusters of 8 in two waves), else 2 up to 148.  Small grids lack
+// the wide levels that pay for the cluster's barriers: one scenario of 600 buses takes 757 us with
+// 8 CTAs and 831 with one, 300 buses 616 and 602; two CTAs gain from 2,000 buses on (38 groups:
+// 2,837 / 3,004 us; at 1,200 buses 1,820 / 1,774).  A batch that shares the GPU with concurrent ones
+// (dense_fused) takes two at most: four parts of 16 groups each took 26.5, 26.0, 28.6 and 37.2 ms
+// with 1, 2, 4 and 8.
+int level_ctas(int groups, int nb, int dense_fused) {
+    if (!dense_fused && nb >= 600)
+        for (int nc : {8, 4})
+            if (groups * nc <= 128) return nc;
+    return nb >= 1600 && groups * 2 <= 148 ? 2 : 1;
 }
 
 int check_launch() {
@@ -893,8 +898,10 @@ int gapk_nr_batch_create(gapk_nr_plan p, int n_scen, const gapk_nr_batch_options
     auto const& h = p->h;
     const size_t G = (n_scen + lanes - 1) / lanes;
     b->G = static_cast<int>(G);
-    b->level_ctas = level_ctas(b->G, b->dense_fused);
-    b->dense_ctas = level_ctas(b->G * lanes, b->dense_fused);
+    b->level_ctas = level_ctas(b->G, h.nb, b->dense_fused);
+    // the dense tail's solves: clusters of small CTAs, no more of them than blocks of 32 rows
+    for (int nc = 8; nc > 1 && b->dense_ctas == 1; nc /= 2)
+        if (!b->dense_fused && (long)G * lanes * nc <= 148 && 32 * nc <= 2 * h.n_tail + 31) b->dense_ctas = nc;
     b->split_slots = b->level_ctas >= 4 ? b->level_ctas * b->threads / lanes : 0;
     const size_t L = G * lanes;
     const size_t esz = b->precision == GAPK_PREC_FP64 ? 8 : 4;
@@ -1352,7 +1359,7 @@ struct gapk_nr_mix_s {
                 int alone;
                 ~Shared() { b->level_ctas = alone; }
             } shared{b, b->level_ctas};
-            b->level_ctas = std::min(b->level_ctas, level_ctas(groups, 0));
+            b->level_ctas = std::min(b->level_ctas, level_ctas(groups, b->plan->h.nb, 0));
             b->cur_refine = ins[i].refine;
             cudaError_t e = cudaStreamBeginCaptureToGraph(cs, graph, nullptr, nullptr, 0,
                                                           cudaStreamCaptureModeThreadLocal);
