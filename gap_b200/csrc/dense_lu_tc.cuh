@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256, 2) k_dense_lu_tc(BatchDev B, int N) {
 
 // The split path's trailing update on the tensor cores (FP32): one CTA per (128 x 128 tile of
 // the trailing block, scenario) for the 32-column panel at k0 (its L21 and U12 written by
-// k_dlu_panel), the tile computed as in k_dense_lu_tc -- operands staged hi / lo, 12 MMAs of the
+// k_dlu_solves), the tile computed as in k_dense_lu_tc -- operands staged hi / lo, 12 MMAs of the
 // transposed product into tensor memory, C loaded while they run, C - D written back from
 // tcgen05.ld registers.  Many CTAs per SM overlap one another's phases.  64 KB of operands, so
 // at most three CTAs share an SM (3 x 128 tensor-memory columns); with k_dense_lu_tc's CTAs on

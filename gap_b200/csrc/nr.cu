@@ -559,10 +559,12 @@ int default_threads(int nb, int lanes) {
 // the wide levels that pay for the cluster's barriers: one scenario of 600 buses takes 757 us with
 // 8 CTAs and 831 with one, 300 buses 616 and 602; two CTAs gain from 2,000 buses on (38 groups:
 // 2,837 / 3,004 us; at 1,200 buses 1,820 / 1,774).  A batch that shares the GPU with concurrent ones
-// (dense_fused) takes two at most: four parts of 16 groups each took 26.5, 26.0, 28.6 and 37.2 ms
-// with 1, 2, 4 and 8.
+// (dense_fused, four of them in the benchmark's pipeline) takes two where four such batches fit:
+// four parts of 16 groups each took 26.5, 26.0, 28.6 and 37.2 ms with 1, 2, 4 and 8, four of 32
+// groups 42.2 and 44.6 ms with 1 and 2.
 int level_ctas(int groups, int nb, int dense_fused) {
-    if (!dense_fused && nb >= 600)
+    if (dense_fused) groups *= 4;
+    else if (nb >= 600)
         for (int nc : {8, 4})
             if (groups * nc <= 128) return nc;
     return nb >= 1600 && groups * 2 <= 148 ? 2 : 1;
@@ -659,7 +661,8 @@ int validate_inputs(gapk_nr_batch b, const gapk_nr_inputs* in) {
 SmallRun small_choice(gapk_nr_batch b, const gapk_nr_inputs* in) {
     auto const& h = b->plan->h;
     SmallRun r;
-    if (b->dev.lvl_ts || b->wait_test || !b->plan->dev.levels) return r;
+    // dense_fused asks for the separate kernels' one-CTA dense LU
+    if (b->dev.lvl_ts || b->wait_test || b->dense_fused || !b->plan->dev.levels) return r;
     const size_t esz = b->precision == GAPK_PREC_FP64 ? 8 : 4;
     r.together = in->refine > 0 && (in->refine_below > 0.0 || in->reuse_below > 0.0);
     long best_cost = 0;
