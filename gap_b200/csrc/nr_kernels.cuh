@@ -1598,7 +1598,9 @@ __global__ void __launch_bounds__(DS_THREADS) k_dense_solve_cl(PlanDev P, BatchD
         const int top = rank + (nblk - 1 - rank) / nc * nc;  // this CTA's last block
         int buf = 0;  // this CTA's next triangle is in tri[buf]
         if (rank < nblk) stage(up ? top : rank, unit, tri[0], rdiag[0], 0);
-        __syncthreads();
+        // a CTA of the cluster must have started before another one writes into its `sol`
+        if (up) __syncthreads();
+        else cta.sync();
         for (int step = 0; step < nblk; ++step) {
             const int b = up ? nblk - 1 - step : step;
             const bool own = b % nc == rank;
