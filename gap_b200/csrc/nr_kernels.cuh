@@ -393,10 +393,11 @@ __global__ void k_check(BatchDev B, int use_cond, cudaGraphConditionalHandle han
                 if (q < B.n_scen && B.solving[q] && B.final_mis[q] < rb) rv = 1;
             }
             // the factors are reused once every iterating lane of the group is below [2];
-            // the solve is then refined against the current FP64 Jacobian
+            // the solve is then refined against the current FP64 Jacobian.  Only factors of this
+            // solve: before its first iteration the batch holds none, or another state's
             const double rf = B.tol[2];
             int fv = 1;
-            if (B.gfactor && rf > 0.0 && sv) {
+            if (B.gfactor && rf > 0.0 && sv && it > 0) {
                 fv = 0;
                 for (int l = 0; l < SW; ++l) {
                     const int q = g * SW + l;

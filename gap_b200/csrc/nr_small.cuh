@@ -498,7 +498,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
             if (together)
                 for (int r = 0; r < parts; ++r) w |= *cg::this_cluster().map_shared_rank(&word[it & 1], r);
             any_iter = w & 2;
-            do_factor = !(below_reuse > 0.0 && (w & 1) && !(w & 8));
+            // (only factors of this solve are reused)
+            do_factor = it == 0 || !(below_reuse > 0.0 && (w & 1) && !(w & 8));
             do_refine = below_refine <= 0.0 || (w & 4) || !do_factor;
         }
         __syncthreads();

@@ -347,7 +347,7 @@ class NRBatch:
         refinement steps only in iterations where a scenario of the lane group has max
         |mismatch| below it.  reuse_below > 0 keeps a group's previous LU factors once all
         its iterating scenarios are below it (the refined solve then corrects against the
-        current Jacobian; needs refine >= 1)."""
+        current Jacobian; needs refine >= 1; a solve's first iteration always factorises)."""
         torch = _torch()
         n = self.plan.info["n_bus"]
         dev = s_spec.device

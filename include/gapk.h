@@ -251,7 +251,8 @@ typedef struct {
     double reuse_below;     /* once every iterating scenario of a lane group has max |mismatch|
                                below this, the group keeps its previous LU factors instead of
                                refactorising, and the (refined, refine >= 1) solve uses them
-                               against the current FP64 Jacobian (0 = refactorise every time) */
+                               against the current FP64 Jacobian (0 = refactorise every time);
+                               a solve's first iteration always factorises                  */
     int v_init_shared;      /* != 0: d_v_init is one start vector [n_bus] for every scenario */
 } gapk_nr_inputs;
 
