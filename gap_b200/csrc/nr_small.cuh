@@ -406,8 +406,8 @@ struct SmallCta {
 
 // One CTA per (lane group, CL of its lanes), from iteration it0 for `passes` iterations (0: until
 // the lanes are done).  State words, voltages, rhs, dx and, on exit, the factors are the ones the
-// separate kernels keep, so every other call on the batch finds them.  With `together` the
-// group's CTAs are one cluster.
+// separate kernels keep, so every other call on the batch finds them (a CTA that factorised nothing
+// leaves the stored factors as they are).  With `together` the group's CTAs are one cluster.
 template <typename T, int CL>
 __global__ void __launch_bounds__(SMALL_THREADS, 4)
     k_nr_small(PlanDev P, BatchDev B, int refine, int together, int passes) {
@@ -450,6 +450,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
     const double tol = B.tol[0];
     const double below_refine = B.A64 ? B.tol[1] : 0.0, below_reuse = B.A64 ? B.tol[2] : 0.0;
     __syncthreads();
+    bool factorised = false;  // by this CTA
     int it = it0;
     for (;; ++it) {
         double m = c.mismatch();
@@ -506,6 +507,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
         if (any_solving) {
             c.jacobian(do_factor, refine > 0 && do_refine);
             __syncthreads();
+            factorised |= do_factor;
             if (do_factor && !c.factor()) singular[lane] = 1;
             c.solve(false);
             if (do_refine) {
@@ -538,9 +540,11 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
     }
     __syncthreads();
     for (int i = c.e0; i < P.n_bus; i += c.ne) B.V[c.at(P.n_bus, i)] = c.v(i);
-    Blk<T>* Fg = reinterpret_cast<Blk<T>*>(B.F);
-    for (int s = c.e0; s < P.n_slots; s += c.ne) stb(Fg + c.at(P.n_slots, s), ldb(c.f(s)));
-    if (N > 0) {
+    if (factorised) {
+        Blk<T>* Fg = reinterpret_cast<Blk<T>*>(B.F);
+        for (int s = c.e0; s < P.n_slots; s += c.ne) stb(Fg + c.at(P.n_slots, s), ldb(c.f(s)));
+    }
+    if (factorised && N > 0) {
         T* Dg = reinterpret_cast<T*>(B.Dt) + (size_t)q * N * dense_ld(N);
         for (int i = c.e0; i < N; i += c.ne)
             for (int j = 0; j < N; ++j)
