@@ -2116,6 +2116,9 @@ __global__ void k_adj_prep(BatchDev B) {
     if (q % SW == 0) {
         B.gsolve[q / SW] = 1;
         B.giter[q / SW] = 1;
+        // refactorised and refined, whatever the last solve's thresholds left here
+        if (B.grefine) B.grefine[q / SW] = 1;
+        if (B.gfactor) B.gfactor[q / SW] = 1;
     }
 }
 
