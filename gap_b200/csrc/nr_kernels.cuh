@@ -219,6 +219,7 @@ __global__ void k_retry_flags(BatchDev B, int policy, int use_cond, cudaGraphCon
         B.ctrl[0] = 0;
         B.ctrl[2] = any;
         B.ctrl[3] = policy;
+        if (any) B.ctrl[4] = 0;  // the retry's loop counts anew
         if (use_cond) cudaGraphSetConditional(handle, any ? 1u : 0u);
     }
 }

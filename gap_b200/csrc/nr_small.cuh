@@ -405,9 +405,10 @@ struct SmallCta {
 };
 
 // One CTA per (lane group, CL of its lanes), from iteration it0 for `passes` iterations (0: until
-// the lanes are done).  State words, voltages, rhs, dx and, on exit, the factors are the ones the
-// separate kernels keep, so every other call on the batch finds them (a CTA that factorised nothing
-// leaves the stored factors as they are).  With `together` the group's CTAs are one cluster.
+// the lanes are done).  State and group words, voltages, rhs, dx and, on exit, the factors are the
+// ones the separate kernels keep, so every other call on the batch finds them (a CTA that factorised
+// nothing leaves the stored factors as they are).  With `together` the group's CTAs are one cluster.
+// A group's giter and gsolve are written by several CTAs: none of them reads these words.
 template <typename T, int CL>
 __global__ void __launch_bounds__(SMALL_THREADS, 4)
     k_nr_small(PlanDev P, BatchDev B, int refine, int together, int passes) {
@@ -418,7 +419,10 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
     __shared__ int any_solving, any_iter, do_factor, do_refine, word[2];
     const SmallLayout L = small_layout(P.n_bus, P.nb, P.n_slots, P.n_tail, P.n_levels, CL, sizeof(T));
     const int parts = B.sw / CL, g = blockIdx.x / parts, tid = threadIdx.x;
-    if (!B.giter[g]) return;
+    bool iterates = false;  // any lane that decides with this CTA's (padding lanes are done)
+    for (int l = 0; l < (together ? B.sw : CL); ++l)
+        iterates |= B.state[g * B.sw + (together ? 0 : blockIdx.x % parts * CL) + l] == 0;
+    if (!iterates) return;
     const int lane = tid % CL, gl = (blockIdx.x % parts) * CL + lane, q = g * B.sw + gl;
     const int N = 2 * P.n_tail;
     const SmallCta<T, CL> c{P, B, (int)L.v, (int)L.x, (int)L.dx, (int)L.d, (int)L.lv, lane, tid / CL,
@@ -556,6 +560,15 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
         B.singular[q] = singular[tid];
     }
     if (tid == 0) {
+        // the words of the last k_check; gsolve is 0 before a stepped pass and 1 before a whole
+        // solve, whose CTAs collect theirs in bit 1
+        if (any_solving) atomicOr(&B.gsolve[g], 2);
+        if (!passes) {
+            atomicAnd(&B.gsolve[g], ~1);
+            B.giter[g] = 0;
+        }
+        if (B.grefine) B.grefine[g] = do_refine;
+        if (B.gfactor) B.gfactor[g] = do_factor;
         if (passes) {
             if (any_iter) atomicOr(&B.ctrl[2], 1);  // k_small_step advances the other words
         } else {
@@ -567,11 +580,12 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
     if (together) cg::this_cluster().sync();  // a neighbour may still read this CTA's word
 }
 
-// Around one stepped pass: before it ([2] any iterating = 0), after it (the iteration count and
-// which groups still iterate).
+// Around one stepped pass: before it ([2] any iterating and each group's gsolve = 0), after it (the
+// iteration count and which groups still iterate).
 __global__ void k_small_step(BatchDev B, int after) {
     if (!after) {
         if (threadIdx.x == 0) B.ctrl[2] = 0;
+        for (int g = threadIdx.x; g < B.n_groups; g += blockDim.x) B.gsolve[g] = 0;
         return;
     }
     for (int g = threadIdx.x; g < B.n_groups; g += blockDim.x) {
