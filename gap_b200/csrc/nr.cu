@@ -546,11 +546,14 @@ struct StateOp {
 };
 
 // CTA size of the level-scheduled kernels where the caller leaves it open: a thread for every
-// eighth (node, lane), which takes all but the widest levels in one round.  3,001 buses x 333
-// scenarios (42 groups): 8.0 ms with 256 threads, 4.6 ms with 1024.
-int default_threads(int nb, int lanes) {
+// eighth (node, lane), which takes all but the widest levels in one round, while the 1,024 threads
+// that their registers allow on an SM still hold all groups at once.  Whole solves with 256 / 512 /
+// 1024 threads, 8 lanes: 3,001 buses, 42 groups 8.0 / - / 4.6 ms; 2,000 buses in FP32, 148 groups
+// 5.74 / 4.59 / 4.06, 149 groups 5.95 / 4.81 / 5.77, 296 groups 7.82 / 6.73 / 7.81, 297 groups 7.97 /
+// 9.02 / 9.44, 592 groups 12.2 / 13.1 / 15.2 ms; the same lines at 1,000 to 10,000 buses and in FP64.
+int default_threads(int nb, int lanes, long groups) {
     int thr = 256;
-    while (thr < 1024 && 8L * thr < (long)nb * lanes) thr *= 2;
+    while (thr < 1024 && 8L * thr < (long)nb * lanes && groups * 2 * thr <= 148 * 1024) thr *= 2;
     return thr;
 }
 // CTAs per lane group of the level-scheduled kernels, one cluster: 8 or 4 where that makes at most
@@ -888,7 +891,7 @@ int gapk_nr_batch_create(gapk_nr_plan p, int n_scen, const gapk_nr_batch_options
     }
     b->sw = lanes;
     int thr = opt ? opt->threads : 0;
-    if (thr == 0) thr = default_threads(p->h.nb, lanes);
+    if (thr == 0) thr = default_threads(p->h.nb, lanes, (n_scen + lanes - 1) / lanes);
     if (thr < 32 || thr > 1024 || thr % 32) {
         set_error("gapk_nr_batch_create: threads must be a multiple of 32 in [32, 1024]");
         return GAPK_EINVAL;
