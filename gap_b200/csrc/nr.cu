@@ -551,10 +551,20 @@ struct StateOp {
 // 1024 threads, 8 lanes: 3,001 buses, 42 groups 8.0 / - / 4.6 ms; 2,000 buses in FP32, 148 groups
 // 5.74 / 4.59 / 4.06, 149 groups 5.95 / 4.81 / 5.77, 296 groups 7.82 / 6.73 / 7.81, 297 groups 7.97 /
 // 9.02 / 9.44, 592 groups 12.2 / 13.1 / 15.2 ms; the same lines at 1,000 to 10,000 buses and in FP64.
+// Past 592 groups the CTAs shrink by the same rule: 500 buses in FP32 with 64 / 96 / 128 / 160 / 192 /
+// 256 threads, 740 groups 5.05 / 4.37 / 3.99 / 3.80 / 3.76 / 4.99 ms, 888 groups 5.39 / 4.72 / 4.36 /
+// 4.17 / 4.43 / 5.34, 2,368 groups 9.4 / 10.8 / 10.0 / 11.2 / 11.4 / 11.9; where not even 64 threads
+// hold them, 128 (3,000 groups: 13.9 / 12.8 / 13.4 / 13.1 / 14.5 / 16.2; in FP64 14.3 / 14.5 / 13.4 /
+// 14.2 / 15.1 / 15.4).  From 1,600 buses on 64 threads are too few for a level (2,000 buses, 1,481
+// groups: 32.5 / 31.8 / 32.8 / 30.8 / 30.9 / 30.9).
 int default_threads(int nb, int lanes, long groups) {
     int thr = 256;
     while (thr < 1024 && 8L * thr < (long)nb * lanes && groups * 2 * thr <= 148 * 1024) thr *= 2;
-    return thr;
+    if (groups * 256 <= 148 * 1024) return thr;
+    for (int t : {192, 160, 128, 96})
+        if (groups <= 148 * (1024 / t)) return t;
+    if (nb >= 1600) return 160;
+    return groups * 64 <= 148 * 1024 ? 64 : 128;
 }
 // CTAs per lane group of the level-scheduled kernels, one cluster: 8 or 4 where that makes at most
 // 128 CTAs (16 clusters of 8 sit on the GPCs side by side; 18 groups of a 2,000-bus grid took 2.2 ms

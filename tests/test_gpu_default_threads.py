@@ -5,10 +5,11 @@ pytestmark = pytest.mark.gpu
 BASE = 1e8
 
 
-@pytest.mark.parametrize("n,scen,precision", [(500, 4096, "fp64"), (1000, 4096, "fp32")])
-def test_many_groups_keep_small_ctas(n, scen, precision):
-    """512 groups: the default is as fast as 256 threads (larger CTAs, which leave the groups to
-    several waves, took 1.28 and 1.36 times as long)."""
+@pytest.mark.parametrize("n,scen,precision,few", [(500, 4096, "fp64", 256), (1000, 4096, "fp32", 256),
+                                                  (500, 5920, "fp32", 192)])
+def test_many_groups_keep_small_ctas(n, scen, precision, few):
+    """512 and 740 groups: the default is as fast as the threads that hold all groups on the GPU at
+    once (larger CTAs, which leave the groups to several waves, take 1.28 to 1.36 times as long)."""
     import torch
 
     from gap_b200 import synth
@@ -25,7 +26,7 @@ def test_many_groups_keep_small_ctas(n, scen, precision):
               policy="newton")
     if precision == "fp32":
         kw.update(refine=2, refine_below=1e-2, reuse_below=1e-2)
-    batches = [NRBatch(plan, scen, precision=precision, threads=t) for t in (0, 256)]
+    batches = [NRBatch(plan, scen, precision=precision, threads=t) for t in (0, few)]
     best = [float("inf")] * 2
     for _ in range(6):
         for i, b in enumerate(batches):
