@@ -78,35 +78,37 @@ __device__ __forceinline__ double2 row_pair(const double* __restrict__ row, int 
     return make_double2(row[c], row[c + 1]);
 }
 
-// One CTA per run of whole rows of at most YB_SLOTS slots and YB_SCEN scenarios, one thread per
+// One CTA per run of whole rows of at most YB_SLOTS slots and NS scenarios, one thread per
 // slot.  Every off-diagonal slot is one end of one branch: its thread computes the branch's
 // stamps once per scenario and leaves the end's diagonal stamp in shared memory, where the
 // diagonal slot's thread sums its row's ends in the reference's order (diag_pos: the slot each
 // end's stamp sits in, or -(s + 1) for shunt s).  Tapped branches (a sine, a cosine and four more
 // divisions) are collected first, from all the CTA's scenarios, and worked off by consecutive
 // threads, so that a warp with one of them does not carry its 31 plain neighbours through that
-// code and the CTA waits for it once per YB_SCEN scenarios.
+// code and the CTA waits for it once per NS scenarios.
 // Bound by the L1 wavefronts of the 48-byte row gathers (67 % busy; FP64 pipe 16 %, DRAM 25 %).
 // 512 scenarios x 38,000 slots (0.66 GB compulsory), with taps / without: 669 / 479 us with the
 // stamps recomputed for every slot and diagonal term, 467 / 350 with one scenario per CTA, 362 /
 // 287 with four; the off-diagonal values kept in registers instead of `val` spill (401 / 297).
-constexpr int YB_SLOTS = 256, YB_SCEN = 4;
+// NS is 4 where that still leaves the GPU several waves of CTAs, 1 up to YB_FEW of those: there a
+// CTA's own chain is the time.  With taps, one scenario of 50 / 1,000 / 10,000 / 30,000 buses 5.5 /
+// 6.4 / 7.1 / 10.5 us with NS = 4, 3.9 / 4.5 / 4.6 / 5.8 with 1; 3,000 buses x 16 (736 CTAs) 9.0 / 6.8,
+// 1,000 x 64 (1,024) 9.4 / 9.4, 10,000 x 12 (1,824) 12.2 / 14.3.
+constexpr int YB_SLOTS = 256, YB_SCEN = 4, YB_FEW = 1024;
 
-template <bool VEC>
+template <bool VEC, int NS>
 __global__ void __launch_bounds__(YB_SLOTS)
-    k_ybus(int n_scen, int n_tiles, const int* __restrict__ tile_row,
-           const int* __restrict__ row_ptr, const int* __restrict__ slot_src,
+    k_ybus(int n_scen, int n_tiles, const int* __restrict__ tile_slot, const int* __restrict__ slot_src,
            const int* __restrict__ diag_ptr, const int* __restrict__ diag_src,
            const int* __restrict__ diag_pos, const double* __restrict__ br, long long br_stride,
            const double* __restrict__ sh, long long sh_stride, int mode, double scale,
            double2* __restrict__ out, long long out_stride) {
-    __shared__ double2 val[YB_SCEN][YB_SLOTS], end[YB_SCEN][YB_SLOTS];
-    __shared__ short tapped[YB_SCEN * YB_SLOTS];  // scenario << 8 | slot
+    __shared__ double2 val[NS][YB_SLOTS], end[NS][YB_SLOTS];
+    __shared__ short tapped[NS * YB_SLOTS];  // scenario << 8 | slot
     __shared__ int n_tapped;
     const int tile = blockIdx.x % n_tiles;
-    const int s0 = (blockIdx.x / n_tiles) * YB_SCEN, s1 = min(n_scen, s0 + YB_SCEN);
-    const int r0 = tile_row[tile], p0 = row_ptr[r0];
-    const int cnt = row_ptr[tile_row[tile + 1]] - p0;
+    const int s0 = (blockIdx.x / n_tiles) * NS, s1 = min(n_scen, s0 + NS);
+    const int p0 = tile_slot[tile], cnt = tile_slot[tile + 1] - p0;
     const int t = threadIdx.x;
     const bool taps = mode != GAPK_YBUS_REFERENCE;
     auto put = [&](int s, int p, double2 v) {
@@ -147,16 +149,16 @@ __global__ void __launch_bounds__(YB_SLOTS)
     __syncthreads();
     if (t < cnt && src >= 0) {
         const double* row = br + (size_t)(src >> 1) * 6;
-        double2 rx[YB_SCEN], gb[YB_SCEN], kt[YB_SCEN];
+        double2 rx[NS], gb[NS], kt[NS];
 #pragma unroll
-        for (int k = 0; k < YB_SCEN; ++k) {
+        for (int k = 0; k < NS; ++k) {
             const double* q = row + (size_t)min(s0 + k, s1 - 1) * br_stride;
             rx[k] = row_pair<VEC>(q, 0);
             gb[k] = row_pair<VEC>(q, 2);
             if (taps) kt[k] = row_pair<VEC>(q, 4);
         }
 #pragma unroll
-        for (int k = 0; k < YB_SCEN; ++k) {
+        for (int k = 0; k < NS; ++k) {
             const SeriesStamp q = series_stamp(rx[k].x, rx[k].y, gb[k].x, gb[k].y);
             end[k][t] = make_double2(q.er, q.ei);
             val[k][t] = make_double2(-q.yr, -q.yi);
@@ -179,17 +181,17 @@ __global__ void __launch_bounds__(YB_SLOTS)
     if (t >= cnt) return;
     if (src >= 0) {
 #pragma unroll
-        for (int k = 0; k < YB_SCEN; ++k)
+        for (int k = 0; k < NS; ++k)
             if (s0 + k < s1) put(s0 + k, t, val[k][t]);
         return;
     }
-    double2 v[YB_SCEN];
+    double2 v[NS];
 #pragma unroll
-    for (int k = 0; k < YB_SCEN; ++k) v[k] = make_double2(0.0, 0.0);
+    for (int k = 0; k < NS; ++k) v[k] = make_double2(0.0, 0.0);
     for (int c = diag_ptr[-src - 1]; c < diag_ptr[-src]; ++c) {
         const int d = diag_pos[c];
 #pragma unroll
-        for (int k = 0; k < YB_SCEN; ++k) {
+        for (int k = 0; k < NS; ++k) {
             double2 a;
             if (d >= 0) {
                 a = end[k][d - p0];
@@ -201,7 +203,7 @@ __global__ void __launch_bounds__(YB_SLOTS)
         }
     }
 #pragma unroll
-    for (int k = 0; k < YB_SCEN; ++k)
+    for (int k = 0; k < NS; ++k)
         if (s0 + k < s1) put(s0 + k, t, v[k]);
 }
 
@@ -277,26 +279,25 @@ using namespace gapk;
 struct gapk_ybus_s {
     YbusPatternHost h;
     int device = -1;
-    std::vector<int> tile_row;  // first row of each CTA's run of rows, then n_bus
+    std::vector<int> tile_slot; // first slot of each CTA's run of rows, then nnz
     std::vector<int> diag_pos;  // diag_src with each branch end replaced by its slot
-    void* d_tile_row = nullptr;
-    void* d_row_ptr = nullptr;
+    void* d_tile_slot = nullptr;
     void* d_diag_pos = nullptr;
     void* d_slot_src = nullptr;
     void* d_diag_ptr = nullptr;
     void* d_diag_src = nullptr;
     ~gapk_ybus_s() {
-        for (void* p : {d_tile_row, d_row_ptr, d_diag_pos, d_slot_src, d_diag_ptr, d_diag_src})
+        for (void* p : {d_tile_slot, d_diag_pos, d_slot_src, d_diag_ptr, d_diag_src})
             if (p) cudaFree(p);
     }
     // Runs of whole rows of at most YB_SLOTS slots (a longer row is a run of its own), and the
     // slot of every branch end.
     void tile() {
-        tile_row.assign(1, 0);
+        tile_slot.assign(1, 0);
         for (int r = 0; r < h.n_bus; ++r)
-            if (r > tile_row.back() && h.row_ptr[r + 1] - h.row_ptr[tile_row.back()] > YB_SLOTS)
-                tile_row.push_back(r);
-        if (h.n_bus > 0) tile_row.push_back(h.n_bus);
+            if (h.row_ptr[r] > tile_slot.back() && h.row_ptr[r + 1] - tile_slot.back() > YB_SLOTS)
+                tile_slot.push_back(h.row_ptr[r]);
+        if (h.n_bus > 0) tile_slot.push_back(h.nnz);
         std::vector<int> slot_of(2 * static_cast<size_t>(h.n_branch), -1);
         for (int p = 0; p < h.nnz; ++p)
             if (h.slot_src[p] >= 0) slot_of[h.slot_src[p]] = p;
@@ -317,8 +318,7 @@ struct gapk_ybus_s {
         if (e == cudaSuccess) e = up(d_diag_ptr, h.diag_ptr);
         if (e == cudaSuccess) e = up(d_diag_src, h.diag_src);
         if (e == cudaSuccess) e = up(d_diag_pos, diag_pos);
-        if (e == cudaSuccess) e = up(d_row_ptr, h.row_ptr);
-        if (e == cudaSuccess) e = up(d_tile_row, tile_row);
+        if (e == cudaSuccess) e = up(d_tile_slot, tile_slot);
         if (e != cudaSuccess) {
             set_error(std::string("ybus upload: ") + cudaGetErrorString(e));
             return e == cudaErrorMemoryAllocation ? GAPK_ENOMEM : GAPK_ECUDA;
@@ -453,14 +453,17 @@ int gapk_ybus_assemble(gapk_ybus y, int n_scen, const double* d_branch, int64_t 
     if (rc) return rc;
     const long long total = (long long)y->h.nnz * n_scen;
     if (total == 0) return GAPK_OK;
-    const int n_tiles = static_cast<int>(y->tile_row.size()) - 1;
-    const long long blocks = (long long)n_tiles * ((n_scen + YB_SCEN - 1) / YB_SCEN);
+    const int n_tiles = static_cast<int>(y->tile_slot.size()) - 1;
     // 16-byte loads need every branch row on a 16-byte boundary (a row is 48 bytes)
     const bool vec = reinterpret_cast<uintptr_t>(d_branch) % 16 == 0 && branch_stride % 2 == 0;
+    const bool few = (long long)n_tiles * n_scen <= YB_FEW;
+    const int ns = few ? 1 : YB_SCEN;
+    const long long blocks = (long long)n_tiles * ((n_scen + ns - 1) / ns);
     auto in = [](void* p) { return static_cast<const int*>(p); };
-    (vec ? k_ybus<true> : k_ybus<false>)<<<static_cast<unsigned>(blocks), YB_SLOTS, 0,
-                                           static_cast<cudaStream_t>(stream)>>>(
-        n_scen, n_tiles, in(y->d_tile_row), in(y->d_row_ptr), in(y->d_slot_src), in(y->d_diag_ptr),
+    auto kernel = few ? (vec ? k_ybus<true, 1> : k_ybus<false, 1>)
+                      : (vec ? k_ybus<true, YB_SCEN> : k_ybus<false, YB_SCEN>);
+    kernel<<<static_cast<unsigned>(blocks), YB_SLOTS, 0, static_cast<cudaStream_t>(stream)>>>(
+        n_scen, n_tiles, in(y->d_tile_slot), in(y->d_slot_src), in(y->d_diag_ptr),
         in(y->d_diag_src), in(y->d_diag_pos), d_branch, branch_stride, d_shunt, shunt_stride, mode,
         scale, reinterpret_cast<double2*>(d_values), values_stride);
     cudaError_t e = cudaGetLastError();
