@@ -8,6 +8,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -72,12 +73,13 @@ struct gapk_nr_plan_s {
     NRPlanHost h;
     std::vector<int> y_row_ptr, y_col;
     bool general = false;  // the plan of a general LU, not of a Newton solve
-    // device copy (current device at first upload)
+    std::vector<int> a_rec;  // a_records(), made with the plan
+    // device copy (current device at first upload): all lists in one allocation
     bool uploaded = false;
     int device = -1;
-    DevBuf d_yrp, d_ycol, d_bt, d_nob, d_si, d_ss, d_lp, d_fa, d_tg, d_pr, d_fb,
-        d_sc, d_lptr, d_lidx, d_rptr, d_rl, d_arp, d_ar, d_var, d_eq, d_schur, d_aslots, d_arec, d_levels, d_words, d_ell, d_acp, d_ac;
+    DevBuf d_lists;
     PlanDev dev{};
+    const int *var_of_comp = nullptr, *eq_of_comp = nullptr;
 
     // the Jacobian fill's records (jac_block), four ints per block
     std::vector<int> a_records() const {
@@ -95,9 +97,10 @@ struct gapk_nr_plan_s {
     }
 
     // k_nr_small's packed schedule (SmallCta): false when not even one FP32 scenario fits its shared
-    // memory, its 16-bit indices or its tail, and for a general matrix.  Threads per target or row (1, 2 or 4): a pass over two entries costs about 70
-    // cycles of latency, adding up two threads' parts about 45, so the longest row decides where
-    // the level leaves threads idle; a wide level keeps a thread per row.
+    // memory, its 16-bit indices or its tail, and for a general matrix.  Threads per target or row
+    // (1, 2 or 4): a pass over two entries costs about 70 cycles of latency, adding up two threads'
+    // parts about 45, so the longest row decides where the level leaves threads idle; a wide level
+    // keeps a thread per row.
     bool small_schedule(std::vector<int>& rec, std::vector<unsigned>& words,
                         std::vector<unsigned>& ell) const {
         if (general || h.n_slots > 0xffff || h.nb > 0xffff || h.n_tail > SMALL_MAX_TAIL ||
@@ -110,15 +113,16 @@ struct gapk_nr_plan_s {
             for (int r = 0; r < rows; ++r) most = std::max(most, count(r));
             const int ls = rows <= 64 && most > 4 ? 2 : rows <= 128 && most > 2 ? 1 : 0;
             const int s = 1 << ls, longest = (most + 2 * s - 1) / (2 * s);
-            out[0] = (int)(ell.size() / 2);
+            const size_t at = ell.size();
+            out[0] = (int)(at / 2);
             out[1] = longest | ls << 16;
-            for (int m = 0; m < longest; ++m)
-                for (int r = 0; r < rows; ++r)
-                    for (int sub = 0; sub < s; ++sub)
-                        for (int o = 0; o < 2; ++o) {
-                            const int i = (2 * m + o) * s + sub;
-                            ell.push_back(i < count(r) ? word(r, i) : pad);
-                        }
+            ell.resize(at + 2 * (size_t)longest * rows * s, pad);
+            // word i = (2 m + o) s + sub of a row: half o of entry m of its part `sub`
+            for (int r = 0; r < rows; ++r)
+                for (int i = 0, n = count(r); i < n; ++i) {
+                    const int sub = i % s, k = i / s;
+                    ell[at + 2 * (((size_t)(k / 2) * rows + r) * s + sub) + k % 2] = word(r, i);
+                }
         };
         auto pack = [](int lo, int hi) { return (unsigned)lo | (unsigned)hi << 16; };
         const unsigned none = pack(h.n_slots, h.n_slots), no_row = pack(h.n_slots, h.nb);
@@ -161,45 +165,70 @@ struct gapk_nr_plan_s {
         return true;
     }
 
+    // One allocation and one copy for all lists (a 200-bus plan and its one-scenario FP64 batch made
+    // and destroyed: 735 us with an allocation and a copy for each list, 440 so).
     int upload() {
         if (uploaded) return GAPK_OK;
-        int rc = 0;
-        auto up = [&](DevBuf& b, std::vector<int> const& v) {
-            if (!rc) rc = b.upload(v);
-        };
-        up(d_yrp, y_row_ptr);
-        up(d_ycol, y_col);
-        up(d_bt, h.bus_type);
-        up(d_nob, h.node_of_bus);
-        up(d_si, h.slot_info);
-        up(d_ss, h.slot_src);
-        up(d_lp, h.level_ptr);
-        up(d_fa, h.fa_ptr);
-        up(d_tg, h.targets);
-        up(d_pr, h.pairs);
-        up(d_fb, h.fb_ptr);
-        up(d_sc, h.scale);
-        up(d_lptr, h.lptr);
-        up(d_lidx, h.lidx);
-        up(d_rptr, h.rptr);
-        up(d_rl, h.rlist);
-        up(d_arp, h.arow_ptr);
-        up(d_ar, h.arow);
-        up(d_var, h.var_of_comp);
-        up(d_eq, h.eq_of_comp);
-        up(d_schur, h.schur);
-        up(d_aslots, h.a_slots);
-        up(d_arec, a_records());
         std::vector<int> rec;
         std::vector<unsigned> words, ell;
-        if (small_schedule(rec, words, ell)) {
-            up(d_levels, rec);
-            if (!rc) rc = d_words.upload(words);
-            if (!rc) rc = d_ell.upload(ell);
+        std::vector<unsigned char> host;
+        auto lists = [&](auto f) {
+            f(dev.y_row_ptr, y_row_ptr);
+            f(dev.y_col, y_col);
+            f(dev.bus_type, h.bus_type);
+            f(dev.node_of_bus, h.node_of_bus);
+            f(dev.slot_info, h.slot_info);
+            f(dev.slot_src, h.slot_src);
+            f(dev.level_ptr, h.level_ptr);
+            f(dev.fa_ptr, h.fa_ptr);
+            f(dev.targets, h.targets);
+            f(dev.pairs, h.pairs);
+            f(dev.fb_ptr, h.fb_ptr);
+            f(dev.scale, h.scale);
+            f(dev.lptr, h.lptr);
+            f(dev.lidx, h.lidx);
+            f(dev.rptr, h.rptr);
+            f(dev.rlist, h.rlist);
+            f(dev.arow_ptr, h.arow_ptr);
+            f(dev.arow, h.arow);
+            f(dev.acol_ptr, h.acol_ptr);
+            f(dev.acol, h.acol);
+            f(dev.schur, h.schur);
+            f(dev.a_slots, h.a_slots);
+            f(dev.a_rec, a_rec);
+            f(var_of_comp, h.var_of_comp);
+            f(eq_of_comp, h.eq_of_comp);
+            f(dev.levels, rec);
+            f(dev.words, words);
+            f(dev.ell, ell);
+        };
+        auto padded = [](auto const& v) { return (v.size() * 4 + 255) & ~size_t(255); };
+        try {
+            if (!small_schedule(rec, words, ell)) {
+                rec.clear();
+                words.clear();
+                ell.clear();
+            }
+            size_t total = 0;
+            lists([&](auto&, auto const& v) { total += padded(v); });
+            host.resize(total);
+        } catch (std::bad_alloc const&) {
+            set_error("plan upload: host allocation failed");
+            return GAPK_ENOMEM;
         }
-        up(d_acp, h.acol_ptr);
-        up(d_ac, h.acol);
+        size_t off = 0;
+        lists([&](auto&, auto const& v) {
+            if (!v.empty()) std::memcpy(host.data() + off, v.data(), v.size() * 4);
+            off += padded(v);
+        });
+        int rc = d_lists.upload(host);
         if (rc) return rc;
+        off = 0;
+        lists([&](auto& p, auto const& v) {
+            using P = std::remove_reference_t<decltype(p)>;
+            p = v.empty() ? nullptr : reinterpret_cast<P>(d_lists.as<unsigned char>() + off);
+            off += padded(v);
+        });
         cudaGetDevice(&device);
         dev.n_bus = h.n_bus;
         dev.nb = h.nb;
@@ -212,32 +241,6 @@ struct gapk_nr_plan_s {
         dev.ns = h.ns;
         dev.n_tail = h.n_tail;
         dev.n_schur = static_cast<int>(h.schur.size() / 4);
-        dev.schur = d_schur.as<int4>();
-        dev.a_slots = d_aslots.as<int>();
-        dev.a_rec = d_arec.as<int4>();
-        dev.levels = d_levels.as<int4>();
-        dev.words = d_words.as<unsigned>();
-        dev.ell = d_ell.as<uint2>();
-        dev.acol_ptr = d_acp.as<int>();
-        dev.acol = d_ac.as<int2>();
-        dev.y_row_ptr = d_yrp.as<int>();
-        dev.y_col = d_ycol.as<int>();
-        dev.bus_type = d_bt.as<int>();
-        dev.node_of_bus = d_nob.as<int>();
-        dev.slot_info = d_si.as<int4>();
-        dev.slot_src = d_ss.as<int>();
-        dev.level_ptr = d_lp.as<int>();
-        dev.fa_ptr = d_fa.as<int>();
-        dev.targets = d_tg.as<int4>();
-        dev.pairs = d_pr.as<int2>();
-        dev.fb_ptr = d_fb.as<int>();
-        dev.scale = d_sc.as<int2>();
-        dev.lptr = d_lptr.as<int>();
-        dev.lidx = d_lidx.as<int>();
-        dev.rptr = d_rptr.as<int>();
-        dev.rlist = d_rl.as<int2>();
-        dev.arow_ptr = d_arp.as<int>();
-        dev.arow = d_ar.as<int2>();
         uploaded = true;
         return GAPK_OK;
     }
@@ -662,22 +665,22 @@ int validate_inputs(gapk_nr_batch b, const gapk_nr_inputs* in) {
     return GAPK_OK;
 }
 
-// How the one-kernel loop (k_nr_small) runs this batch on these inputs: lanes per CTA (0: the
-// separate kernels are used), CTA size, whether a group's lanes decide together, and the shared
-// memory share of the SM.  Shapes are ranked by waves of CTAs, then by fewer lanes per CTA (a
+// How the one-kernel loop (k_nr_small) runs this batch, with or without per-group refinement or
+// reuse thresholds: lanes per CTA (0: the separate kernels are used), CTA size, whether a group's
+// lanes decide together, and the shared memory share of the SM.  Shapes are ranked by waves of CTAs, then by fewer lanes per CTA (a
 // lane more in a CTA lengthens every step of the level schedule), then by 256 threads over 128.
 // Against the separate kernels on transmission grids of 120 to 1,200 buses it takes 1/1.6 to 1/3
 // of their time while one wave holds the scenarios and 1/1.1 to 1/1.6 with two.  With three it
 // still wins where an SM holds several FP32 CTAs (500 buses x 1024: 1,564 us against 1,610) or one
 // FP64 CTA (900 x 300: 1,507 / 1,583), and loses with several FP64 ones (300 x 1024: 982 / 856) or
 // one FP32 CTA, whose groups wait for each other across SMs (900 x 300: 1,481 / 1,365).
-SmallRun small_choice(gapk_nr_batch b, const gapk_nr_inputs* in) {
+SmallRun small_choice(gapk_nr_batch b, bool thresholds) {
     auto const& h = b->plan->h;
     SmallRun r;
     // dense_fused asks for the separate kernels' one-CTA dense LU
     if (b->dev.lvl_ts || b->wait_test || b->dense_fused || !b->plan->dev.levels) return r;
     const size_t esz = b->precision == GAPK_PREC_FP64 ? 8 : 4;
-    r.together = in->refine > 0 && (in->refine_below > 0.0 || in->reuse_below > 0.0);
+    r.together = thresholds;
     long best_cost = 0;
     for (int cl = 1; cl <= b->sw; cl *= 2) {
         const size_t bytes = small_layout(h.n_bus, h.nb, h.n_slots, h.n_tail, h.n_levels, cl, esz).total;
@@ -698,6 +701,9 @@ SmallRun small_choice(gapk_nr_batch b, const gapk_nr_inputs* in) {
     }
     r.together &= r.cl < b->sw;  // one CTA holds the whole group otherwise
     return r;
+}
+SmallRun small_choice(gapk_nr_batch b, const gapk_nr_inputs* in) {
+    return small_choice(b, in->refine > 0 && (in->refine_below > 0.0 || in->reuse_below > 0.0));
 }
 
 template <typename T, int CL>
@@ -735,17 +741,13 @@ struct DenseSolveAttributesOp {
         if (*e == cudaSuccess) *e = set(k_dense_solve_cl<T, SW, true>);
     }
 };
-template <typename T>
-cudaError_t small_attributes() {
-    auto set = [](auto fn) {
-        return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_SMEM_MAX);
-    };
-    cudaError_t e = set(k_nr_small<T, 1>);
-    if (e == cudaSuccess) e = set(k_nr_small<T, 2>);
-    if (e == cudaSuccess) e = set(k_nr_small<T, 4>);
-    if (e == cudaSuccess) e = set(k_nr_small<T, 8>);
-    return e;
-}
+template <typename T, int CL>
+struct SmallAttributesOp {
+    static void run(cudaError_t* e) {
+        *e = cudaFuncSetAttribute(k_nr_small<T, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)SMALL_SMEM_MAX);
+    }
+};
 
 int load_inputs(gapk_nr_batch b, const gapk_nr_inputs* in, cudaStream_t st) {
     int rc = validate_inputs(b, in);
@@ -792,12 +794,13 @@ int gapk_nr_plan_create(int n_bus, int nnz_y, const int* h_y_row_ptr, const int*
     try {
         if (!analyze_nr(n_bus, nnz_y, h_y_row_ptr, h_y_col_idx, h_bus_type, jac, ord, dmin, p->h))
             return GAPK_EINVAL;
+        p->y_row_ptr.assign(h_y_row_ptr, h_y_row_ptr + n_bus + 1);
+        p->y_col.assign(h_y_col_idx, h_y_col_idx + nnz_y);
+        p->a_rec = p->a_records();
     } catch (std::bad_alloc const&) {
         set_error("gapk_nr_plan_create: host allocation failed");
         return GAPK_ENOMEM;
     }
-    p->y_row_ptr.assign(h_y_row_ptr, h_y_row_ptr + n_bus + 1);
-    p->y_col.assign(h_y_col_idx, h_y_col_idx + nnz_y);
     *out = p.release();
     return GAPK_OK;
 }
@@ -977,8 +980,10 @@ int gapk_nr_batch_create(gapk_nr_plan p, int n_scen, const gapk_nr_batch_options
             return GAPK_ECUDA;
         }
     }
-    if (p->dev.levels) {
-        cudaError_t e = esz == 8 ? small_attributes<double>() : small_attributes<float>();
+    // (the lanes per CTA do not depend on a solve's inputs)
+    if (const SmallRun r = small_choice(b.get(), false); r.cl) {
+        cudaError_t e = cudaSuccess;
+        dispatch_tsw<SmallAttributesOp>(b->precision, r.cl, &e);
         if (e != cudaSuccess) {
             set_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
             return GAPK_ECUDA;
@@ -1162,14 +1167,14 @@ int gapk_nr_adjoint_branch(gapk_nr_batch b, int n_branch, const int* d_from, con
 
 int gapk_nr_stage_get_correction(gapk_nr_batch b, double* d_dx, void* stream) {
     if (!b || !d_dx) return GAPK_EINVAL;
-    dispatch_tsw<ToRefOp>(b->precision, b->sw, b, b->dev.dx, b->plan->d_var.as<int>(),
+    dispatch_tsw<ToRefOp>(b->precision, b->sw, b, b->dev.dx, b->plan->var_of_comp,
                           b->plan->h.n_vars, 1.0, d_dx, static_cast<cudaStream_t>(stream));
     return check_launch();
 }
 
 int gapk_nr_stage_get_mismatch(gapk_nr_batch b, double* d_f, void* stream) {
     if (!b || !d_f) return GAPK_EINVAL;
-    dispatch_tsw<ToRefOp>(b->precision, b->sw, b, b->dev.rhs, b->plan->d_eq.as<int>(),
+    dispatch_tsw<ToRefOp>(b->precision, b->sw, b, b->dev.rhs, b->plan->eq_of_comp,
                           b->plan->h.n_vars, -1.0, d_f, static_cast<cudaStream_t>(stream));
     return check_launch();
 }
@@ -1729,13 +1734,12 @@ extern "C" int gapk_nr_solve_noalloc(gapk_nr_plan p, const gapk_nr_inputs* in,
     }
     auto const& h = p->h;
     const size_t n = h.n_bus, nb = h.nb, nnz = h.nnz_y, N = 2 * (size_t)h.n_tail;
-    const std::vector<int> a_rec = p->a_records();
     // plan index lists copied into the scratch, in this order
     std::vector<int> const* lists[] = {&p->y_row_ptr, &p->y_col, &h.bus_type, &h.node_of_bus,
                                        &h.slot_info, &h.slot_src, &h.level_ptr,
                                        &h.fa_ptr, &h.targets, &h.pairs,
                                        &h.fb_ptr, &h.scale, &h.lptr, &h.lidx, &h.rptr,
-                                       &h.rlist, &h.schur, &a_rec};
+                                       &h.rlist, &h.schur, &p->a_rec};
     constexpr int kLists = sizeof(lists) / sizeof(lists[0]);
     Carver c;
     size_t loff[kLists];
