@@ -304,6 +304,11 @@ template <typename K, typename... A>
 void launch_levels(gapk_nr_batch b, cudaStream_t st, K kernel, A... args) {
     launch_clusters(b->G, b->level_ctas, b->threads, 0, st, kernel, args...);
 }
+template <typename T, int SW>
+void launch_sparse_factor(gapk_nr_batch b, cudaStream_t st) {
+    launch_levels(b, st, b->split_slots ? k_factor<T, SW, true> : k_factor<T, SW, false>, b->plan->dev,
+                  b->dev, b->split_slots);
+}
 // The tail's two substitutions; k_dense_solve streams best when its CTAs fill the GPU.
 template <typename T, int SW, bool TR>
 void launch_dense_solve(gapk_nr_batch b, cudaStream_t st, double2* out, int acc) {
@@ -329,7 +334,7 @@ template <typename T, int SW>
 void launch_factor(gapk_nr_batch b, cudaStream_t st) {
     PlanDev const& P = b->plan->dev;
     BatchDev const& B = b->dev;
-    launch_levels(b, st, k_factor<T, SW>, P, B, b->split_slots);
+    launch_sparse_factor<T, SW>(b, st);
     if (P.n_tail > 0) {
         dim3 gs(blocks_for((long)P.n_schur * SW, 256), b->G);
         k_schur<T, SW><<<gs, 256, 0, st>>>(P, B);
@@ -465,7 +470,7 @@ struct KernelOp {
         switch (which) {
             case 0: k_mismatch<SW><<<mismatch_grid<SW>(P, G), 256, 0, st>>>(P, B); break;
             case 1: k_jfill<T, SW><<<dim3(blocks_for((long)P.n_a * SW, 256), G), 256, 0, st>>>(P, B); break;
-            case 2: launch_levels(b, st, k_factor<T, SW>, P, B, b->split_slots); break;
+            case 2: launch_sparse_factor<T, SW>(b, st); break;
             case 3:
                 if (P.n_tail > 0)
                     k_schur<T, SW><<<dim3(blocks_for((long)P.n_schur * SW, 256), G), 256, 0, st>>>(P, B);
@@ -1858,7 +1863,7 @@ extern "C" int gapk_nr_solve_noalloc(gapk_nr_plan p, const gapk_nr_inputs* in,
         k_mismatch<1><<<mismatch_grid<1>(P, 1), 256, 0, st>>>(P, D);
         k_check<1><<<1, 1024, 0, st>>>(D, 0, cudaGraphConditionalHandle{});
         k_jfill<double, 1><<<blocks_for((long)h.n_a, 256), 256, 0, st>>>(P, D);
-        k_factor<double, 1><<<1, thr, 0, st>>>(P, D, 0);
+        k_factor<double, 1, false><<<1, thr, 0, st>>>(P, D, 0);
         if (h.n_tail > 0) {
             k_schur<double, 1><<<blocks_for((long)P.n_schur, 256), 256, 0, st>>>(P, D);
             launch_dense_lu<double>(dense_w, 1, dense_smem, st, D, (int)N, false);

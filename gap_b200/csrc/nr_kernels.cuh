@@ -556,8 +556,8 @@ __global__ void __launch_bounds__(256) k_jfill(PlanDev P, BatchDev B) {
 struct LevelCta {
     int nc, rank, g;
     __device__ __forceinline__ LevelCta() {
-        asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(nc));
-        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        nc = __clusterSizeInBlocks();
+        rank = __clusterRelativeBlockRank();
         g = blockIdx.x / nc;
     }
     __device__ __forceinline__ void sync() const {
@@ -649,7 +649,10 @@ __device__ __forceinline__ void pair_sum(Blk<T>& acc, const Blk<T>* F, const int
     }
 }
 
-template <typename T, int SW>
+// SPLIT: narrow levels split their targets over split_slots.  Without it the kernel has registers to
+// spare for its two targets in flight: one scenario of 100 / 300 / 1,000 buses in FP64 57 / 68 / 72 us,
+// 62 / 72 / 73 with the split code in it and not taken.
+template <typename T, int SW, bool SPLIT>
 __global__ void __launch_bounds__(1024) k_factor(PlanDev P, BatchDev B, int split_slots) {
     const LevelCta cta;
     const int g = cta.g;
@@ -666,8 +669,8 @@ __global__ void __launch_bounds__(1024) k_factor(PlanDev P, BatchDev B, int spli
     __syncthreads();
     for (int h = 0; h < P.n_levels; ++h) {
         const int ta = fa[h], tb = fa[h + 1];
-        const int ls = split_slots && tb > ta ? min(split_log(tb - ta, split_slots), 5 - SW_LOG) : 0, s = 1 << ls;
-        if (s > 1) {
+        const int ls = SPLIT && tb > ta ? min(split_log(tb - ta, split_slots), 5 - SW_LOG) : 0, s = 1 << ls;
+        if (SPLIT && s > 1) {
             // narrow levels: s neighbouring threads share a target's pairs (the longest lists, 20
             // to 40 pairs, set the level's latency)
             const int sub = e0 & (s - 1), wl = e0 % (32 / SW);
@@ -694,7 +697,7 @@ __global__ void __launch_bounds__(1024) k_factor(PlanDev P, BatchDev B, int spli
         }
         // two targets per worker at a time (targets of one level are independent), so that
         // their gathers overlap in memory
-        for (int t = s > 1 ? tb : ta + e0; t < tb; t += 2 * ne) {
+        for (int t = SPLIT && s > 1 ? tb : ta + e0; t < tb; t += 2 * ne) {
             const bool two = t + ne < tb;
             const int4 tg = P.targets[t];
             const int4 tg2 = two ? P.targets[t + ne] : make_int4(0, 0, 0, 0);
