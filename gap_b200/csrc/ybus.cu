@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <memory>
+#include <new>
 #include <string>
 #include <utility>
 #include <vector>
@@ -279,16 +280,14 @@ using namespace gapk;
 struct gapk_ybus_s {
     YbusPatternHost h;
     int device = -1;
-    std::vector<int> tile_slot; // first slot of each CTA's run of rows, then nnz
-    std::vector<int> diag_pos;  // diag_src with each branch end replaced by its slot
-    void* d_tile_slot = nullptr;
-    void* d_diag_pos = nullptr;
-    void* d_slot_src = nullptr;
-    void* d_diag_ptr = nullptr;
-    void* d_diag_src = nullptr;
+    std::vector<int> tile_slot;  // first slot of each CTA's run of rows, then nnz
+    std::vector<int> diag_pos;   // diag_src with each branch end replaced by its slot
+    // the device's copies, one allocation
+    int* d_lists = nullptr;
+    const int *d_tile_slot = nullptr, *d_slot_src = nullptr, *d_diag_ptr = nullptr,
+              *d_diag_src = nullptr, *d_diag_pos = nullptr;
     ~gapk_ybus_s() {
-        for (void* p : {d_tile_slot, d_diag_pos, d_slot_src, d_diag_ptr, d_diag_src})
-            if (p) cudaFree(p);
+        if (d_lists) cudaFree(d_lists);
     }
     // Runs of whole rows of at most YB_SLOTS slots (a longer row is a run of its own), and the
     // slot of every branch end.
@@ -307,22 +306,30 @@ struct gapk_ybus_s {
     }
     int upload() {
         if (d_slot_src) return GAPK_OK;
-        auto up = [](void*& d, std::vector<int> const& v) -> cudaError_t {
-            size_t bytes = (v.empty() ? 1 : v.size()) * sizeof(int);
-            cudaError_t e = cudaMalloc(&d, bytes);
-            if (e != cudaSuccess) return e;
-            if (!v.empty()) e = cudaMemcpy(d, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice);
-            return e;
-        };
-        cudaError_t e = up(d_slot_src, h.slot_src);
-        if (e == cudaSuccess) e = up(d_diag_ptr, h.diag_ptr);
-        if (e == cudaSuccess) e = up(d_diag_src, h.diag_src);
-        if (e == cudaSuccess) e = up(d_diag_pos, diag_pos);
-        if (e == cudaSuccess) e = up(d_tile_slot, tile_slot);
+        std::vector<int> host;
+        size_t at[5], n = 0;
+        try {
+            for (std::vector<int> const* v : {&tile_slot, &h.slot_src, &h.diag_ptr, &h.diag_src, &diag_pos}) {
+                at[n++] = host.size();
+                host.insert(host.end(), v->begin(), v->end());
+            }
+            host.push_back(0);  // no list starts past the allocation
+        } catch (std::bad_alloc const&) {
+            set_error("ybus upload: host allocation failed");
+            return GAPK_ENOMEM;
+        }
+        cudaError_t e = d_lists ? cudaSuccess : cudaMalloc(&d_lists, host.size() * sizeof(int));
+        if (e == cudaSuccess)
+            e = cudaMemcpy(d_lists, host.data(), host.size() * sizeof(int), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
             set_error(std::string("ybus upload: ") + cudaGetErrorString(e));
             return e == cudaErrorMemoryAllocation ? GAPK_ENOMEM : GAPK_ECUDA;
         }
+        d_tile_slot = d_lists + at[0];
+        d_slot_src = d_lists + at[1];
+        d_diag_ptr = d_lists + at[2];
+        d_diag_src = d_lists + at[3];
+        d_diag_pos = d_lists + at[4];
         cudaGetDevice(&device);
         return GAPK_OK;
     }
@@ -459,13 +466,12 @@ int gapk_ybus_assemble(gapk_ybus y, int n_scen, const double* d_branch, int64_t 
     const bool few = (long long)n_tiles * n_scen <= YB_FEW;
     const int ns = few ? 1 : YB_SCEN;
     const long long blocks = (long long)n_tiles * ((n_scen + ns - 1) / ns);
-    auto in = [](void* p) { return static_cast<const int*>(p); };
     auto kernel = few ? (vec ? k_ybus<true, 1> : k_ybus<false, 1>)
                       : (vec ? k_ybus<true, YB_SCEN> : k_ybus<false, YB_SCEN>);
     kernel<<<static_cast<unsigned>(blocks), YB_SLOTS, 0, static_cast<cudaStream_t>(stream)>>>(
-        n_scen, n_tiles, in(y->d_tile_slot), in(y->d_slot_src), in(y->d_diag_ptr),
-        in(y->d_diag_src), in(y->d_diag_pos), d_branch, branch_stride, d_shunt, shunt_stride, mode,
-        scale, reinterpret_cast<double2*>(d_values), values_stride);
+        n_scen, n_tiles, y->d_tile_slot, y->d_slot_src, y->d_diag_ptr, y->d_diag_src, y->d_diag_pos,
+        d_branch, branch_stride, d_shunt, shunt_stride, mode, scale,
+        reinterpret_cast<double2*>(d_values), values_stride);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error(std::string("k_ybus launch: ") + cudaGetErrorString(e));
