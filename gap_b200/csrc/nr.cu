@@ -309,13 +309,14 @@ void launch_sparse_factor(gapk_nr_batch b, cudaStream_t st) {
     launch_levels(b, st, b->split_slots ? k_factor<T, SW, true> : k_factor<T, SW, false>, b->plan->dev,
                   b->dev, b->split_slots);
 }
-// The tail's two substitutions; k_dense_solve streams best when its CTAs fill the GPU.
+// The tail's two substitutions; k_dense_solve streams best when its CTAs fill the GPU, for tails that
+// fit the 48 KB that any launch gets (order 5,088 in FP64).
 template <typename T, int SW, bool TR>
 void launch_dense_solve(gapk_nr_batch b, cudaStream_t st, double2* out, int acc) {
     PlanDev const& P = b->plan->dev;
     if (P.n_tail == 0) return;
     const size_t smem = dense_solve_smem(P.n_tail, sizeof(T));
-    if (TR || b->dense_ctas > 1)
+    if (TR || b->dense_ctas > 1 || smem + 32 * 33 * sizeof(T) > 48 * 1024)
         launch_clusters(b->G * SW, b->dense_ctas, DS_THREADS, smem, st, k_dense_solve_cl<T, SW, TR>, P, b->dev, out, acc);
     else
         k_dense_solve<T, SW><<<b->G * SW, 256, smem, st>>>(P, b->dev, out, acc);
