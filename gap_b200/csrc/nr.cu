@@ -165,13 +165,15 @@ struct gapk_nr_plan_s {
         return true;
     }
 
-    // One allocation and one copy for all lists (a 200-bus plan and its one-scenario FP64 batch made
-    // and destroyed: 735 us with an allocation and a copy for each list, 440 so).
+    // One allocation for all lists, one copy for those of at most 64 KB (a 200-bus plan and its
+    // one-scenario FP64 batch made and destroyed: 735 us with an allocation and a copy for each list,
+    // 440 so).  Larger lists are copied from where they are: collecting them too costs more than their
+    // copies' calls.
     int upload() {
         if (uploaded) return GAPK_OK;
         std::vector<int> rec;
         std::vector<unsigned> words, ell;
-        std::vector<unsigned char> host;
+        std::vector<unsigned char> host;  // the small lists, the allocation's front
         auto lists = [&](auto f) {
             f(dev.y_row_ptr, y_row_ptr);
             f(dev.y_col, y_col);
@@ -202,33 +204,44 @@ struct gapk_nr_plan_s {
             f(dev.words, words);
             f(dev.ell, ell);
         };
-        auto padded = [](auto const& v) { return (v.size() * 4 + 255) & ~size_t(255); };
+        // f(pointer, list, offset, small)
+        size_t front = 0, total = 0;
+        auto each = [&](auto f) {
+            size_t at[2] = {front, 0};  // of the next large, small list
+            lists([&](auto& p, auto const& v) {
+                const size_t bytes = v.size() * 4;
+                const bool small = bytes <= 64 * 1024;
+                f(p, v, at[small], small);
+                at[small] += (bytes + 255) & ~size_t(255);
+            });
+            total = at[0];
+            return at[1];
+        };
         try {
             if (!small_schedule(rec, words, ell)) {
                 rec.clear();
                 words.clear();
                 ell.clear();
             }
-            size_t total = 0;
-            lists([&](auto&, auto const& v) { total += padded(v); });
-            host.resize(total);
+            front = each([](auto&, auto const&, size_t, bool) {});
+            host.resize(front);
         } catch (std::bad_alloc const&) {
             set_error("plan upload: host allocation failed");
             return GAPK_ENOMEM;
         }
-        size_t off = 0;
-        lists([&](auto&, auto const& v) {
-            if (!v.empty()) std::memcpy(host.data() + off, v.data(), v.size() * 4);
-            off += padded(v);
+        each([&](auto&, auto const& v, size_t at, bool small) {
+            if (small && !v.empty()) std::memcpy(host.data() + at, v.data(), v.size() * 4);
         });
-        int rc = d_lists.upload(host);
+        int rc = d_lists.alloc(total);
         if (rc) return rc;
-        off = 0;
-        lists([&](auto& p, auto const& v) {
+        cudaError_t e = cudaMemcpy(d_lists.p, host.data(), front, cudaMemcpyHostToDevice);
+        each([&](auto& p, auto const& v, size_t at, bool small) {
             using P = std::remove_reference_t<decltype(p)>;
-            p = v.empty() ? nullptr : reinterpret_cast<P>(d_lists.as<unsigned char>() + off);
-            off += padded(v);
+            unsigned char* d = d_lists.as<unsigned char>() + at;
+            p = v.empty() ? nullptr : reinterpret_cast<P>(d);
+            if (!small && e == cudaSuccess) e = cudaMemcpy(d, v.data(), v.size() * 4, cudaMemcpyHostToDevice);
         });
+        GAPK_CUDA_TRY(e);
         cudaGetDevice(&device);
         dev.n_bus = h.n_bus;
         dev.nb = h.nb;
