@@ -556,10 +556,11 @@ __global__ void __launch_bounds__(256) k_jfill(PlanDev P, BatchDev B) {
 struct LevelCta {
     int nc, rank, g;
     __device__ __forceinline__ LevelCta() {
-        nc = __clusterSizeInBlocks();
-        rank = __clusterRelativeBlockRank();
+        asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(nc));
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
         g = blockIdx.x / nc;
     }
+    __device__ __forceinline__ LevelCta(int nc, int rank) : nc(nc), rank(rank), g(blockIdx.x / nc) {}
     __device__ __forceinline__ void sync() const {
         if (nc == 1) {
             __syncthreads();
@@ -654,7 +655,9 @@ __device__ __forceinline__ void pair_sum(Blk<T>& acc, const Blk<T>* F, const int
 // 62 / 72 / 73 with the split code in it and not taken.
 template <typename T, int SW, bool SPLIT>
 __global__ void __launch_bounds__(1024) k_factor(PlanDev P, BatchDev B, int split_slots) {
-    const LevelCta cta;
+    // read again where they are used, which frees two registers; the sweeps, with registers to spare,
+    // are faster with the values kept (10,000 buses x 1024: 0.32 against 0.35 ms)
+    const LevelCta cta(__clusterSizeInBlocks(), __clusterRelativeBlockRank());
     const int g = cta.g;
     if (!B.gsolve[g] || (B.gfactor && !B.gfactor[g])) return;
     __shared__ int fa_buf[LV_MAX + 1], fb_buf[LV_MAX + 1];
