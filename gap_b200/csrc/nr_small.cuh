@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
     __shared__ double red[SMALL_THREADS / 32][CL];
     __shared__ double mis[CL];
     __shared__ int state[CL], solving[CL], singular[CL];
-    __shared__ int any_solving, any_iter, do_factor, do_refine, word[2];
+    __shared__ int any_solving, any_iter, do_factor, do_refine, factorised, word[2];
     const SmallLayout L = small_layout(P.n_bus, P.nb, P.n_slots, P.n_tail, P.n_levels, CL, sizeof(T));
     const int parts = B.sw / CL, g = blockIdx.x / parts, tid = threadIdx.x;
     bool iterates = false;  // any lane that decides with this CTA's (padding lanes are done)
@@ -434,6 +434,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
         stb(c.f(P.n_slots), Blk<T>{0, 0, 0, 0});
         stv(c.x(P.nb), Vec2<T>{0, 0});
     }
+    if (tid == 0) factorised = 0;
     if (tid < CL) {
         state[tid] = B.state[q];
         solving[tid] = B.solving[q];
@@ -454,7 +455,6 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
     const double tol = B.tol[0];
     const double below_refine = B.A64 ? B.tol[1] : 0.0, below_reuse = B.A64 ? B.tol[2] : 0.0;
     __syncthreads();
-    bool factorised = false;  // by this CTA
     int it = it0;
     for (;; ++it) {
         double m = c.mismatch();
@@ -505,13 +505,13 @@ __global__ void __launch_bounds__(SMALL_THREADS, 4)
             any_iter = w & 2;
             // (only factors of this solve are reused)
             do_factor = it == 0 || !(below_reuse > 0.0 && (w & 1) && !(w & 8));
+            if (any_solving && do_factor) factorised = 1;  // by this CTA
             do_refine = below_refine <= 0.0 || (w & 4) || !do_factor;
         }
         __syncthreads();
         if (any_solving) {
             c.jacobian(do_factor, refine > 0 && do_refine);
             __syncthreads();
-            factorised |= do_factor;
             if (do_factor && !c.factor()) singular[lane] = 1;
             c.solve(false);
             if (do_refine) {
