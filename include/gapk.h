@@ -211,11 +211,15 @@ typedef struct {
     int precision;      /* GAPK_PREC_*                                                     */
     int y_shared;       /* 1: one Y for all scenarios; 0: one Y per scenario               */
     int lanes;          /* scenarios interleaved per thread group: 1, 2, 4 or 8 (0 = auto) */
-    int threads;        /* threads per CTA of the factor / solve kernels (0 = auto)        */
-    int use_graph;      /* 1: NR loop as a CUDA graph with a device-side while node        */
-    int dense_fused;    /* 1: one-CTA-per-scenario dense-tail LU even for a batch too small
-                           to fill the GPU alone (batches that run concurrently on several
-                           streams); 0: chosen by the batch size                           */
+    int threads;        /* threads per CTA of the level-scheduled factor / solve kernels
+                           (0 = auto; the one-kernel loop of small grids has its own size)  */
+    int use_graph;      /* 1: NR loop as a CUDA graph with a device-side while node; 0: driven
+                           by the host (the one-kernel loop of small grids needs neither)   */
+    int dense_fused;    /* 1: the batch runs concurrently with others on several streams: one-
+                           CTA-per-scenario dense-tail LU even where the batch is too small to
+                           fill the GPU alone, clusters of CTAs sized for four such batches,
+                           no clustered dense solves and no one-kernel loop for a small grid;
+                           0: all chosen by this batch's size                              */
     int dense_fma;      /* FP32 tails have the trailing updates of their dense LU on the tensor
                            cores (tcgen05, three TF32 products accumulated in FP32:
                            k_dense_lu_tc one CTA per scenario, k_dlu_update_tc on the split
@@ -223,6 +227,10 @@ typedef struct {
                            use CUDA cores.                                                   */
 } gapk_nr_batch_options;
 
+/* A batch repeats its results bit for bit.  Across batches a scenario's last bits may differ with
+ * the number of scenarios beside it, also on grids without a dense tail: sums are split over
+ * threads by the batch's shape, and that number chooses between the one-kernel loop of small
+ * grids and the separate kernels. */
 int gapk_nr_batch_create(gapk_nr_plan p, int n_scen, const gapk_nr_batch_options* opt,
                          gapk_nr_batch* out);
 int gapk_nr_batch_destroy(gapk_nr_batch b);
